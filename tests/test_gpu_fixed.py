@@ -1,0 +1,83 @@
+"""The fixed-point form of the FP64 path at the edges of its range, against the
+CPU oracle.  Tolerance: the path's 1e-9 max(1, |lnL|), times (1 - e)^-2, by
+which both sides' column errors grow near pericentre."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import oracle_lnl, synth_chunk, synth_star
+
+pytestmark = pytest.mark.gpu
+
+
+def _lnl(star, chunk, jitter):
+    from thejoker_gb300 import device as dev
+    table = dev.StarTable([star], jitter="applied" if jitter else "reference")
+    cache = dev.PriorCache.from_samples(chunk)
+    out = torch.empty((1, len(chunk)), dtype=torch.float64, device="cuda")
+    dev.lnl(table, cache, out, precision="fp64")
+    return out[0].cpu().numpy()
+
+
+def _check(star, chunk, jitter):
+    got, ref = _lnl(star, chunk, jitter), oracle_lnl(star, chunk, jitter)
+    tol = 1e-9 * np.maximum(1.0, np.abs(ref)) / (1.0 - chunk[:, 1]) ** 2
+    assert np.all(np.abs(got - ref) <= tol)
+
+
+@pytest.mark.parametrize("jitter", [False, True])
+@pytest.mark.parametrize("N,poly,noff", [(1, 1, 0), (3, 1, 0), (33, 2, 1), (256, 1, 0),
+                                         (257, 3, 1), (530, 2, 0), (40, 3, 2)])
+def test_epochs_and_columns(cuda, N, poly, noff, jitter):
+    rng = np.random.default_rng(100 * N + poly)
+    star = synth_star(rng, N, poly=poly, noff=min(noff, 1), t0=0.0)
+    if noff == 2:                            # six linear parameters
+        star["trend_M"] = np.hstack([star["trend_M"], (star["t"] > 500.0)[:, None] * 1.0])
+        star["mu"], star["lam"] = np.zeros(6), np.append(star["lam"], 4.0)
+    chunk = synth_chunk(rng, 129 if N < 100 else 12, jitter=jitter)
+    chunk[:, 1] = np.minimum(chunk[:, 1], 0.9)
+    _check(star, chunk, jitter)
+
+
+@pytest.mark.parametrize("jitter", [False, True])
+def test_sample_edges(cuda, jitter):
+    """Eccentricities and jitters on both sides of the lines, tiny and huge
+    periods, angles of either sign, times before the reference."""
+    rng = np.random.default_rng(7)
+    star = synth_star(rng, 20, t0=0.0)
+    star["t_ref"] = 400.0
+    chunk = synth_chunk(rng, 96, jitter=jitter)
+    chunk[:, 1] = np.minimum(chunk[:, 1], 0.9)
+    chunk[:8, 1] = [0.0, 1e-300, 1e-9, 3e-6, 0.99, 0.999, 0.99900001, 0.9995]
+    chunk[8:12, 0] = [1e-3, 1e5, 1e9, 2.0 ** -22]
+    chunk[12:16, 3] = [-3.0, 40.0, 0.0, 2000.0]
+    chunk[16:20, 2] = [-3.0, 40.0, 0.0, 2000.0]
+    if jitter:
+        chunk[20:26, 4] = [0.0, 1e-8, 1e2, 1e5, 2e5, 1e9]
+    phase = np.abs(1000.0 / chunk[:, 0])     # turns: a double's phase is good to 2^-52 of them
+    keep = phase < 1e6
+    got, ref = _lnl(star, chunk, jitter), oracle_lnl(star, chunk, jitter)
+    tol = 1e-9 * np.maximum(1.0, np.abs(ref)) / (1.0 - chunk[:, 1]) ** 2
+    assert np.all((np.abs(got - ref) <= tol)[keep]) and np.all(np.isfinite(got))
+
+
+@pytest.mark.parametrize("ratio", [255.0, 257.0, 1e8])
+@pytest.mark.parametrize("jitter", [False, True])
+def test_weight_spans(cuda, ratio, jitter):
+    rng = np.random.default_rng(8)
+    star = synth_star(rng, 12, poly=2, t0=0.0)
+    star["ivar"] = 1.0 / np.geomspace(1.0, ratio, 12)
+    chunk = synth_chunk(rng, 64, jitter=jitter)
+    chunk[:, 1] = np.minimum(chunk[:, 1], 0.9)
+    _check(star, chunk, jitter)
+
+
+def test_prior_mean(cuda):
+    """A K prior mean other than zero: the jitter form runs in doubles."""
+    rng = np.random.default_rng(9)
+    star = synth_star(rng, 12, t0=0.0)
+    star["mu"] = np.array([5.0, 1.0])
+    for jitter in (False, True):
+        chunk = synth_chunk(rng, 64, jitter=jitter)
+        chunk[:, 1] = np.minimum(chunk[:, 1], 0.9)
+        _check(star, chunk, jitter)

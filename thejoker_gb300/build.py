@@ -21,7 +21,7 @@ SOURCES = ["joker_lnl.cu", "joker_lnl_packed.cu", "joker_lnl_fast.cu", "joker_ln
            "joker_noalloc.cu", "joker_iter.cu", "joker_posterior.cu", "joker_prior.cu"]
 HEADERS = ["joker_internal.cuh", "joker_math.cuh", "joker_fp64.cuh", "joker_mixed.cuh",
            "joker_fast.cuh",
-           "joker_sincos_table.cuh"]
+           "joker_sincos_table.cuh", "joker_fixed.cuh", "joker_trig_table.cuh"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2"]
 

@@ -14,6 +14,7 @@
 #include <mutex>
 #include <tuple>
 #include "joker_internal.cuh"
+#include "joker_fixed.cuh"
 
 namespace joker {
 cudaError_t launch_lnl(int precision, int L, bool jit, const LnlArgs &a, int block,
@@ -159,6 +160,57 @@ static bool spd_inverse(int n, const long double *A, long double *Ainv, long dou
         for (int i = 0; i < n; ++i) Ainv[i * n + c] = col[i];
     }
     return true;
+}
+
+// The fixed-point form of a star's FP64 epoch records (fx::EpochFx): powers of
+// two that bring times, weights, velocities and trend columns to 62 bits.
+// A star has one when its weights span at most 2^8 -- each then keeps the 53
+// bits of a double -- and its values are far from the ends of a double's range.
+static void prep_fixed(int n, int L, StarRec &r, double *rec64) {
+    auto expo = [](double v) { int e = 0; std::frexp(v, &e); return e; };   // |v| < 2^e
+    double tm = 0.0, ym = 0.0, wm = 0.0, wl = INFINITY, Tm[MAXL] = {0.0};
+    for (int i = 0; i < n; ++i) {
+        const double *q = rec64 + (size_t)i * REC64;
+        tm = std::max(tm, std::fabs(q[0]));
+        ym = std::max(ym, std::fabs(q[1]));
+        wm = std::max(wm, q[2]);
+        wl = std::min(wl, q[2]);
+        for (int j = 2; j < L; ++j) {
+            if (!(std::fabs(q[2 + j]) <= 0x1p200)) return;
+            Tm[j] = std::max(Tm[j], std::fabs(q[2 + j]));
+        }
+    }
+    if (!(tm <= 0x1p60 && ym <= 0x1p200 && wm <= 0x1p200 && wl >= 0x1p-200 && wm <= 256.0 * wl))
+        return;
+    auto scale = [&](double v) { return std::max(expo(v), -200); };        // 0: any scale
+    const int et = std::max(expo(tm), -400), ew = scale(wm), ey = scale(ym);
+    r.fx_tsh = 62 - et;
+    r.fx_w = std::ldexp(1.0, ew);
+    r.fx_y = std::ldexp(1.0, ey);
+    auto fixed = [](double v, int sh) { return (int64_t)std::llrint(std::ldexp(v, sh)); };
+    auto limb = [](int64_t v) {
+        const int64_t lim = ((int64_t)1 << 62) - 1;                        // |v| < 1 may round up
+        return fx::split(std::min(std::max(v, -lim), lim));
+    };
+    int64_t t0 = INT64_MAX;
+    for (int i = 0; i < n; ++i) t0 = std::min(t0, fixed(rec64[(size_t)i * REC64], r.fx_tsh));
+    r.fx_t0 = t0;
+    int eT[MAXL] = {0};
+    for (int j = 2; j < L; ++j) {
+        eT[j] = scale(Tm[j]);
+        r.fx_T[j] = std::ldexp(1.0, eT[j]);
+    }
+    for (int i = 0; i < n; ++i) {
+        double *q = rec64 + (size_t)i * REC64;
+        fx::EpochFx f;
+        memset(&f, 0, sizeof f);
+        f.t = (uint64_t)(fixed(q[0], r.fx_tsh) - t0);
+        f.w = limb(fixed(q[2], 62 - ew));
+        f.y = limb(fixed(q[1], 62 - ey));
+        for (int j = 2; j < L; ++j) f.T[j - 2] = limb(fixed(q[2 + j], 62 - eT[j]));
+        memcpy(q + FX64, &f, sizeof f);
+    }
+    r.fx_ok = 1;
 }
 
 // Per-star preparation on the host, in FP64 / long double: the StarRec
@@ -386,6 +438,7 @@ static int prep_star(int k, int L, int jitter_mode, int n, const double *t, cons
     r.phase_c = (float)(rms * (2.0L * 3.141592653589793238462643383279502884L * 2.5L *
                                0x1p-34L * (1.0L + 1e-6L)));
     for (int j = 1; j < L; ++j) r.Wjj[j] = (float)(Wjj[j] * (1.0L + 1e-6L));
+    prep_fixed(n, L, r, rec64);
     return JOKER_OK;
 }
 
@@ -763,7 +816,7 @@ extern "C" int joker_batch_marginal_ln_likelihood(const joker_stars *s, int star
     a.row0 = 0;
     a.count = n_samples;
     a.ld = n_samples;
-    a.chunk = 1024;
+    a.chunk = 128;
     a.ips = (n_samples + a.chunk - 1) / a.chunk;
     a.n_items = (int)std::min<int64_t>(a.ips, INT32_MAX);
     if (a.ips > INT32_MAX) return fail(JOKER_ERANGE, "n_samples too large for one call");

@@ -3,6 +3,7 @@
 #pragma once
 #include "joker_internal.cuh"
 #include "joker_math.cuh"
+#include "joker_fixed.cuh"
 
 namespace joker {
 
@@ -260,9 +261,179 @@ __device__ __forceinline__ double Acc64<L, JIT>::finish(const StarRec &st, doubl
     }
 }
 
-// FP64 ln L of one sample with the star's epochs read from global memory.
+// Per-sample state of the fixed-point form: the integer epoch sums, and the
+// same finish as Acc64's from their doubles.  Sums of integers do not depend
+// on the order, so every split of the epochs over threads gives the same ln L.
+//
+// With the jitter the weights are w_j = 2^ew g wn_j, g = 1 / (1 + a),
+// a = s^2 2^ew, wn_j = v_j / d_j, v_j = ivar_j 2^-ew and
+// d_j = v_j + g (1 - v_j) in [v_j, 1], and
+// sum log(1 + s^2 ivar_j) = sum log d_j + n log(1 + a).
 template <int L, bool JIT>
-__device__ __noinline__ double fp64_lnl_global(const StarRec &st, const double *ep64, double P,
+struct AccFx {
+    fx::Orbit orb;
+    fx::Sum96 A00, b0, A0[MAXL];             // no jitter; jitter: G00, q0, G0k
+    fx::Sum96 G[L][L], q[L], rWr;            // jitter: the rest
+    fx::limbs g62;
+    double g, a;
+    int64_t pj;                              // prod d_j = pj 2^(ej - 62)
+    int ej;
+
+    // False: the sample (or star) needs the FP64 form.
+    __device__ __forceinline__ bool init(const StarRec &st, double P, double e, double om,
+                                         double M0, double s) {
+        A00.zero();
+        b0.zero();
+#pragma unroll
+        for (int k = 0; k < MAXL; ++k) A0[k].zero();
+        if (JIT) {
+#pragma unroll
+            for (int i = 0; i < L; ++i) {
+                q[i].zero();
+#pragma unroll
+                for (int k = 0; k < L; ++k) G[i][k].zero();
+            }
+            rWr.zero();
+            pj = fx::ONE62 - 1;
+            ej = 0;
+            a = s * s * st.fx_w;
+            if (!(st.mu0 == 0.0 && a <= 0x1p40)) return false;
+            g = rcp_newton(1.0 + a);
+            g62 = fx::split(fx::fixed62(g));
+        }
+        return st.fx_ok && orb.init(st.fx_tsh, st.fx_t0, P, e, om, M0);
+    }
+
+    __device__ __forceinline__ void add(const fx::EpochFx &r) {
+        const int64_t mq = orb.column(r.t);                            // Q61
+        const fx::limbs m = fx::split(mq);
+        if (!JIT) {
+            const int64_t wmq = fx::mul(r.w, m);                       // Q61
+            const fx::limbs wm = fx::split(wmq);
+            A00.add(fx::mul(wm, m));                                   // Q60
+            b0.add(fx::mul(wm, r.y));                                  // Q61
+            if (L > 1) A0[1].add(wmq);                                 // Q61; T_1 = 1
+#pragma unroll
+            for (int k = 2; k < L; ++k) A0[k].add(fx::mul(wm, r.T[k - 2]));
+        } else {
+            const int64_t v = fx::join(r.w);
+            const int64_t d = fx::clamp62(v + fx::mul(g62, fx::split(fx::ONE62 - v)));
+            const int64_t wq = fx::twice(fx::div61(v >> 1, d >> 1));   // Q62
+            pj = fx::mul(fx::split(pj), fx::split(d));
+            const int z = fx::clz64((uint64_t)pj) - 2;
+            pj <<= z;
+            ej -= z;
+            const fx::limbs w = fx::split(wq);
+            const int64_t wmq = fx::mul(w, m), wyq = fx::mul(w, r.y);
+            const fx::limbs wm = fx::split(wmq), wy = fx::split(wyq);
+            A00.add(fx::mul(wm, m));                                   // Q60
+            b0.add(fx::mul(wm, r.y));                                  // Q61
+            rWr.add(fx::mul(wy, r.y));                                 // Q62
+            if (L > 1) {
+                A0[1].add(wmq);                                        // Q61
+                G[1][1].add(wq);                                       // Q62
+                q[1].add(wyq);                                         // Q62
+            }
+#pragma unroll
+            for (int i = 2; i < L; ++i) {
+                const int64_t wTq = fx::mul(w, r.T[i - 2]);
+                const fx::limbs wT = fx::split(wTq);
+                A0[i].add(fx::mul(wm, r.T[i - 2]));                    // Q61
+                G[i][1].add(wTq);                                      // Q62
+                q[i].add(fx::mul(wy, r.T[i - 2]));                     // Q62
+#pragma unroll
+                for (int k = 2; k <= i; ++k) G[i][k].add(fx::mul(wT, r.T[k - 2]));
+            }
+        }
+    }
+
+    // Over the 32 lanes of a warp (every lane gets the totals).
+    __device__ __forceinline__ void warp_sum() {
+        A00.warp_sum();
+        b0.warp_sum();
+#pragma unroll
+        for (int k = 1; k < L; ++k) A0[k].warp_sum();
+        if (JIT) {
+            rWr.warp_sum();
+#pragma unroll
+            for (int i = 1; i < L; ++i) {
+                q[i].warp_sum();
+#pragma unroll
+                for (int k = 1; k <= i; ++k) G[i][k].warp_sum();
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const int64_t p2 = (int64_t)__shfl_xor_sync(0xffffffffu, (unsigned long long)pj, o);
+                ej += __shfl_xor_sync(0xffffffffu, ej, o);
+                pj = fx::mul(fx::split(pj), fx::split(p2));
+                const int z = fx::clz64((uint64_t)pj) - 2;
+                pj <<= z;
+                ej -= z;
+            }
+        }
+    }
+
+    // The jitter form's sums as doubles: the lower triangle of M W M^T, M W y
+    // and y W y.
+    __device__ __forceinline__ void system(const StarRec &st, double (&Gd)[L][L], double (&qd)[L],
+                                           double &yy) const {
+        const double c = st.fx_w * g;
+        Gd[0][0] = A00.value() * (c * 0x1p-60);
+        qd[0] = b0.value() * (c * st.fx_y * 0x1p-61);
+        yy = rWr.value() * (c * st.fx_y * st.fx_y * 0x1p-62);
+#pragma unroll
+        for (int i = 1; i < L; ++i) {
+            const double ti = i == 1 ? c : c * st.fx_T[i];
+            Gd[i][0] = A0[i].value() * (ti * 0x1p-61);
+            qd[i] = q[i].value() * (ti * st.fx_y * 0x1p-62);
+#pragma unroll
+            for (int k = 1; k <= i; ++k)
+                Gd[i][k] = G[i][k].value() * ((k == 1 ? ti : ti * st.fx_T[k]) * 0x1p-62);
+        }
+    }
+
+    // sum log(1 + s^2 ivar_j) less log of the returned factor in [1/2, 1)
+    __device__ __forceinline__ double log_rest(const StarRec &st, double &factor) const {
+        factor = (double)pj * 0x1p-62;
+        return fma((double)ej, 0.69314718055994530942, (double)st.n_epochs * log1p(a));
+    }
+
+    __device__ __forceinline__ double finish(const StarRec &st, double P, double e) const {
+        const double lam0 = k_prior_variance(st, P, e);
+        if constexpr (!JIT) {
+            double Ad[MAXL];
+#pragma unroll
+            for (int k = 1; k < L; ++k)
+                Ad[k] = A0[k].value() * ((k == 1 ? st.fx_w : st.fx_w * st.fx_T[k]) * 0x1p-61);
+            return tail_schur_d<L, false>(st, A00.value() * (st.fx_w * 0x1p-60), Ad,
+                                          b0.value() * (st.fx_w * st.fx_y * 0x1p-61), lam0, 0.0);
+        } else {
+            double Gd[L][L], qd[L], yy, f;
+            system(st, Gd, qd, yy);
+            const double ilam0 = st.k_scaled ? rcp_newton(lam0) : st.ilam[0];
+#pragma unroll
+            for (int i = 0; i < L; ++i) Gd[i][i] += i == 0 ? ilam0 : st.ilam[i];
+            const double lr = log_rest(st, f);
+            return tail_full_d<L, false>(Gd, qd, yy, st.log_norm_rest - st.sum_log_ivar + lr,
+                                         lam0 * f);
+        }
+    }
+};
+
+// An epoch's fixed-point record, from global memory.
+__device__ __forceinline__ fx::EpochFx load_epoch_fx(const double *rec) {
+    fx::EpochFx r;
+    const int4 *src = reinterpret_cast<const int4 *>(rec + FX64);
+    int4 *dst = reinterpret_cast<int4 *>(&r);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) dst[k] = __ldg(src + k);
+    return r;
+}
+
+// FP64 ln L of one sample with the star's epochs read from global memory, in
+// doubles: the form for what the fixed-point one does not take.
+template <int L, bool JIT>
+__device__ __noinline__ double fp64_lnl_doubles(const StarRec &st, const double *ep64, double P,
                                                double e, double om, double M0, double s) {
     Acc64<L, JIT> acc;
     acc.init(st, P, e, om, M0, s);
@@ -276,17 +447,37 @@ __device__ __noinline__ double fp64_lnl_global(const StarRec &st, const double *
     return acc.finish(st, P);
 }
 
+// FP64 ln L of one sample with the star's epochs read from global memory.
+template <int L, bool JIT>
+__device__ __noinline__ double fp64_lnl_global(const StarRec &st, const double *ep64, double P,
+                                               double e, double om, double M0, double s) {
+    AccFx<L, JIT> acc;
+    if (acc.init(st, P, e, om, M0, s)) {
+        const double *rec = ep64 + (size_t)st.epoch_off * REC64;
+        for (int i = 0; i < st.n_epochs; ++i, rec += REC64) acc.add(load_epoch_fx(rec));
+        if (!acc.orb.bad) return acc.finish(st, P, e);
+    }
+    return fp64_lnl_doubles<L, JIT>(st, ep64, P, e, om, M0, s);
+}
+
 // FP64 ln L of one sample evaluated by a whole warp: lane l takes epochs l,
 // l + 32, ...; the sums are combined across the warp.  All 32 lanes must call
-// it with the same sample; all return the value.  Same arithmetic per epoch
-// as fp64_lnl_global, summed in a different order (agreement to FP64
-// rounding of the sums).
+// it with the same sample; all return the value.  The fixed-point form gives
+// fp64_lnl_global's number; the FP64 form sums in a different order (agreement
+// to FP64 rounding of the sums).
 template <int L, bool JIT>
 __device__ __noinline__ double fp64_lnl_warp_t(const StarRec &st, const double *ep64, double P,
                                                double e, double om, double M0, double s) {
+    const double *rec0 = ep64 + (size_t)st.epoch_off * REC64;
+    AccFx<L, JIT> fxa;
+    if (fxa.init(st, P, e, om, M0, s)) {
+        for (int i = threadIdx.x & 31; i < st.n_epochs; i += 32)
+            fxa.add(load_epoch_fx(rec0 + (size_t)i * REC64));
+        fxa.warp_sum();
+        if (!__any_sync(0xffffffffu, fxa.orb.bad)) return fxa.finish(st, P, e);
+    }
     Acc64<L, JIT> acc;
     acc.init(st, P, e, om, M0, s);
-    const double *rec0 = ep64 + (size_t)st.epoch_off * REC64;
     for (int i = threadIdx.x & 31; i < st.n_epochs; i += 32) {
         const double *rec = rec0 + (size_t)i * REC64;
         double T[MAXL];

@@ -13,7 +13,8 @@ constexpr int MAXL = JOKER_MAX_LINEAR;
 void count_launch();
 constexpr int TILE = 256;          // epochs staged in shared memory at a time
 constexpr int REC32 = 20;          // floats per epoch record of the mixed kernel
-constexpr int REC64 = 8;           // doubles per epoch record of the FP64 kernel
+constexpr int REC64 = 16;          // doubles per FP64 epoch record: 8 doubles, then the
+constexpr int FX64 = 8;            // fixed-point form (fx::EpochFx) from double 8 on
 constexpr int MAX_CK = 8;          // early-exit checkpoints per star (fused pass)
 
 // Per-star constants, built on the host in FP64 (joker_abi.cu).  Index 0 of
@@ -75,6 +76,12 @@ struct alignas(16) StarRec {
     int32_t ck_k[MAX_CK];
     float ck[MAX_CK][8];          // P1, P2, C + kappa, Hi11, Hi12, Hi22, log det H, 0
     float ck_full[8];             // the same over all epochs (P = 0, C + kappa = chi2_0)
+    // Fixed-point form of the FP64 path: whether the star has one, the time
+    // unit 2^-fx_tsh days, the integer time fx_t0 of the first epoch, and the
+    // powers of two by which weights, velocities and trend columns are scaled.
+    int32_t fx_ok, fx_tsh;
+    int64_t fx_t0;
+    double fx_w, fx_y, fx_T[MAXL];
 };
 
 // One unit of the persistent likelihood kernels: `count` samples of star
