@@ -56,6 +56,7 @@ struct joker_stars {
     int slot_epochs = 0;         // > 0 for a slot table (joker_stars_create_slots)
     int64_t total_epochs = 0;
     std::vector<int64_t> off;
+    std::vector<unsigned char> fixed;   // per star: see stars_fixed
     StarRec *d_stars = nullptr;
     double *d_ep64 = nullptr;
     float *d_ep32 = nullptr;
@@ -495,6 +496,7 @@ extern "C" int joker_stars_create(joker_stars **out, int n_stars, int n_linear,
     s->max_epochs = max_ep;
     s->total_epochs = NE;
     s->off.assign(epoch_offsets, epoch_offsets + n_stars + 1);
+    for (const StarRec &r : recs) s->fixed.push_back(r.fx_ok && r.mu0 == 0.0);
     auto cleanup = [&]() { joker_stars_destroy(s); };
     cudaError_t e;
     if ((e = cudaMalloc(&s->d_stars, sizeof(StarRec) * n_stars)) != cudaSuccess ||
@@ -543,6 +545,7 @@ extern "C" int joker_stars_create_slots(joker_stars **out, int n_slots, int max_
     s->slot_epochs = max_epochs;
     s->total_epochs = (int64_t)n_slots * max_epochs;
     s->off.resize(n_slots + 1);
+    s->fixed.assign(n_slots, 0);
     for (int k = 0; k <= n_slots; ++k) s->off[k] = (int64_t)k * max_epochs;
     std::vector<StarRec> recs(n_slots);
     memset(recs.data(), 0, sizeof(StarRec) * n_slots);
@@ -596,6 +599,7 @@ extern "C" int joker_stars_set(joker_stars *s, int slot, int n_epochs, const dou
     CUDA_TRY(cudaMemcpyAsync(s->d_ep32 + (size_t)r.epoch_off * REC32, r32.data(),
                              sizeof(float) * r32.size(), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(s->d_stars + slot, &r, sizeof(StarRec), cudaMemcpyHostToDevice, st));
+    s->fixed[slot] = r.fx_ok && r.mu0 == 0.0;
     // pageable sources: staged before the calls return
     return JOKER_OK;
 }
@@ -789,7 +793,9 @@ extern "C" int joker_cache_load(joker_cache *c, const double *d_chunk, int64_t n
 // ---------------------------------------------------------------- likelihood
 static int run_lnl(const joker_stars *s, int precision, LnlArgs a, int block,
                    cudaStream_t st) {
-    CUDA_TRY(cudaMemsetAsync(s->d_queue, 0, sizeof(int), st));
+    // the FP64 kernel takes its items by block
+    if (precision != JOKER_FP64) CUDA_TRY(cudaMemsetAsync(s->d_queue, 0, sizeof(int), st));
+    a.max_epochs = s->max_epochs;
     CUDA_TRY(launch_lnl(precision, s->L, s->jitter == JOKER_JITTER_APPLIED, a, block, st));
     return JOKER_OK;
 }
@@ -838,6 +844,11 @@ void stars_internals(const joker_stars *s, const StarRec **recs, const double **
     *jit = s->jitter == JOKER_JITTER_APPLIED;
     *queue = s->d_queue;
 }
+
+int stars_max_epochs(const joker_stars *s) { return s->max_epochs; }
+// whether the star's records have the fixed-point form and its K prior mean is
+// zero, as that form's full system wants
+bool stars_fixed(const joker_stars *s, int star) { return s->fixed[star] != 0; }
 
 void cache_internals(const joker_cache *c, int64_t *cap, const double **P, const double **E,
                      const double **OM, const double **M0, const double **S, int64_t *stride,

@@ -230,12 +230,13 @@ __device__ __forceinline__ double tail_full_d(const double (&G)[L][L], const dou
     return -0.5 * (rWr - quad + logdet);
 }
 
-// K prior variance per sample (fast_likelihood.pyx:461-464)
-__device__ __forceinline__ double k_prior_variance(const StarRec &st, double P, double e) {
+// K prior variance per sample (fast_likelihood.pyx:461-464; clip: at max_K^2)
+__device__ __forceinline__ double k_prior_variance(const StarRec &st, double P, double e,
+                                                   bool clip = true) {
     if (!st.k_scaled) return st.lam0;
     const double y = rcbrt_newton(P * st.iP0);                  // (P / P0)^(-1/3)
     const double v = st.sigK0sq * (y * y) * rcp_newton(1.0 - e * e);
-    return fmin(st.maxK2, v);
+    return clip ? fmin(st.maxK2, v) : v;
 }
 
 template <int L, bool JIT>
@@ -319,10 +320,7 @@ struct AccFx {
             const int64_t v = fx::join(r.w);
             const int64_t d = fx::clamp62(v + fx::mul(g62, fx::split(fx::ONE62 - v)));
             const int64_t wq = fx::twice(fx::div61(v >> 1, d >> 1));   // Q62
-            pj = fx::mul(fx::split(pj), fx::split(d));
-            const int z = fx::clz64((uint64_t)pj) - 2;
-            pj <<= z;
-            ej -= z;
+            times(d, 0);
             const fx::limbs w = fx::split(wq);
             const int64_t wmq = fx::mul(w, m), wyq = fx::mul(w, r.y);
             const fx::limbs wm = fx::split(wmq), wy = fx::split(wyq);
@@ -347,29 +345,75 @@ struct AccFx {
         }
     }
 
-    // Over the 32 lanes of a warp (every lane gets the totals).
-    __device__ __forceinline__ void warp_sum() {
-        A00.warp_sum();
-        b0.warp_sum();
+    // f on every sum
+    template <class F> __device__ __forceinline__ void each(F f) {
+        f(A00);
+        f(b0);
 #pragma unroll
-        for (int k = 1; k < L; ++k) A0[k].warp_sum();
+        for (int k = 1; k < L; ++k) f(A0[k]);
         if (JIT) {
-            rWr.warp_sum();
+            f(rWr);
 #pragma unroll
             for (int i = 1; i < L; ++i) {
-                q[i].warp_sum();
+                f(q[i]);
 #pragma unroll
-                for (int k = 1; k <= i; ++k) G[i][k].warp_sum();
+                for (int k = 1; k <= i; ++k) f(G[i][k]);
             }
+        }
+    }
+    static constexpr int SUMS = 1 + L + (JIT ? L + L * (L - 1) / 2 : 0);
+    static constexpr int WORDS = 3 * SUMS + 1 + (JIT ? 3 : 0);           // of a stored state
+
+    __device__ __forceinline__ void times(int64_t p2, int e2) {
+        pj = fx::mul(fx::split(pj), fx::split(p2));
+        const int z = fx::clz64((uint64_t)pj) - 2;
+        pj <<= z;
+        ej += e2 - z;
+    }
+
+    // Over the 32 lanes of a warp (every lane gets the totals).
+    __device__ __forceinline__ void warp_sum() {
+        each([](fx::Sum96 &v) { v.warp_sum(); });
+        if (JIT) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 const int64_t p2 = (int64_t)__shfl_xor_sync(0xffffffffu, (unsigned long long)pj, o);
-                ej += __shfl_xor_sync(0xffffffffu, ej, o);
-                pj = fx::mul(fx::split(pj), fx::split(p2));
-                const int z = fx::clz64((uint64_t)pj) - 2;
-                pj <<= z;
-                ej -= z;
+                times(p2, __shfl_xor_sync(0xffffffffu, ej, o));
             }
+        }
+    }
+
+    // The sums as WORDS words, 32 apart, and the sum with such a state.
+    __device__ __forceinline__ void store(uint32_t *w) {
+        int k = 0;
+        auto put = [&](uint32_t v) { w[32 * k++] = v; };
+        each([&](fx::Sum96 &v) {
+            put((uint32_t)v.lo);
+            put((uint32_t)(v.lo >> 32));
+            put((uint32_t)v.hi);
+        });
+        put((uint32_t)orb.bad);
+        if (JIT) {
+            put((uint32_t)pj);
+            put((uint32_t)((uint64_t)pj >> 32));
+            put((uint32_t)ej);
+        }
+    }
+    __device__ __forceinline__ void merge(const uint32_t *w) {
+        int k = 0;
+        auto get = [&]() { return w[32 * k++]; };
+        auto get64 = [&]() {
+            const uint32_t l = get();
+            return ((uint64_t)get() << 32) | l;
+        };
+        each([&](fx::Sum96 &v) {
+            const int64_t l = (int64_t)get64();
+            v.add(l, (int32_t)get());
+        });
+        orb.bad |= (int32_t)get();
+        if (JIT) {
+            const int64_t p2 = (int64_t)get64();
+            times(p2, (int32_t)get());
         }
     }
 
@@ -392,6 +436,16 @@ struct AccFx {
         }
     }
 
+    // No jitter: the K row A00, A0k of M W M^T and K's entry b0 of M W y.
+    __device__ __forceinline__ void k_row(const StarRec &st, double &a00, double &b,
+                                          double *a0) const {
+        a00 = A00.value() * (st.fx_w * 0x1p-60);
+        b = b0.value() * (st.fx_w * st.fx_y * 0x1p-61);
+#pragma unroll
+        for (int k = 1; k < L; ++k)
+            a0[k] = A0[k].value() * ((k == 1 ? st.fx_w : st.fx_w * st.fx_T[k]) * 0x1p-61);
+    }
+
     // sum log(1 + s^2 ivar_j) less log of the returned factor in [1/2, 1)
     __device__ __forceinline__ double log_rest(const StarRec &st, double &factor) const {
         factor = (double)pj * 0x1p-62;
@@ -401,12 +455,9 @@ struct AccFx {
     __device__ __forceinline__ double finish(const StarRec &st, double P, double e) const {
         const double lam0 = k_prior_variance(st, P, e);
         if constexpr (!JIT) {
-            double Ad[MAXL];
-#pragma unroll
-            for (int k = 1; k < L; ++k)
-                Ad[k] = A0[k].value() * ((k == 1 ? st.fx_w : st.fx_w * st.fx_T[k]) * 0x1p-61);
-            return tail_schur_d<L, false>(st, A00.value() * (st.fx_w * 0x1p-60), Ad,
-                                          b0.value() * (st.fx_w * st.fx_y * 0x1p-61), lam0, 0.0);
+            double a00, b, a0[MAXL];
+            k_row(st, a00, b, a0);
+            return tail_schur_d<L, false>(st, a00, a0, b, lam0, 0.0);
         } else {
             double Gd[L][L], qd[L], yy, f;
             system(st, Gd, qd, yy);
@@ -428,6 +479,61 @@ __device__ __forceinline__ fx::EpochFx load_epoch_fx(const double *rec) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) dst[k] = __ldg(src + k);
     return r;
+}
+
+// The fixed-point halves of n FP64 epoch records, into shared memory.
+__device__ __forceinline__ void stage_epochs_fx(fx::EpochFx *sm, const double *src, int n) {
+    const int4 *s4 = reinterpret_cast<const int4 *>(src + FX64);
+    int4 *d4 = reinterpret_cast<int4 *>(sm);
+    for (int i = threadIdx.x; i < n * 4; i += blockDim.x)
+        d4[i] = __ldg(s4 + (i >> 2) * (REC64 / 2) + (i & 3));
+}
+
+// A block of 128 threads works on 128 / S samples, S = 1, 2 or 4: warp w takes
+// every S-th epoch, from w % S on, of the 32 samples of group w / S, and the
+// states meet in the group's first warp.  S > 1 is for calls whose samples
+// alone leave SMs idle or the last wave short.
+constexpr int SLICED_BLOCK = 128;
+
+// Shared memory of such a block: a tile of epochs, then the stored states.
+template <int L, bool JIT> constexpr int sliced_smem(int S) {
+    const int tile = TILE * (int)sizeof(fx::EpochFx);
+    const int states = (4 / S) * (S - 1) * AccFx<L, JIT>::WORDS * 128;
+    return tile > states ? tile : states;
+}
+
+// All epochs of a star into the samples' states; afterwards the first warp of
+// each group holds the totals (true there).  `go`: this thread's sample takes
+// the fixed-point form.  Called by the whole block.
+template <int L, bool JIT>
+__device__ __forceinline__ bool sliced_epochs(AccFx<L, JIT> &acc, bool go, const StarRec &st,
+                                              const double *ep64, void *smem, int S) {
+    fx::EpochFx *sm = static_cast<fx::EpochFx *>(smem);
+    const int warp = threadIdx.x >> 5, slice = warp & (S - 1), N = st.n_epochs;
+    for (int t0 = 0; t0 < N; t0 += TILE) {
+        const int nt = min(TILE, N - t0);
+        __syncthreads();
+        stage_epochs_fx(sm, ep64 + ((size_t)st.epoch_off + t0) * REC64, nt);
+        __syncthreads();
+        if (go)
+            for (int i = (slice - t0) & (S - 1); i < nt; i += S) acc.add(sm[i]);
+    }
+    if (S == 1) return true;
+    __syncthreads();
+    uint32_t *w = static_cast<uint32_t *>(smem) +
+                  ((warp / S) * (S - 1) * AccFx<L, JIT>::WORDS) * 32 + (threadIdx.x & 31);
+    if (slice > 0) acc.store(w + (slice - 1) * AccFx<L, JIT>::WORDS * 32);
+    __syncthreads();
+    if (slice == 0)
+        for (int k = 0; k < S - 1; ++k) acc.merge(w + k * AccFx<L, JIT>::WORDS * 32);
+    return slice == 0;
+}
+
+// S for n samples of at most N epochs: four while the 128-sample blocks would
+// be fewer than four waves of the 608 that 152 SMs hold (a last wave of one
+// block in four costs most of a wave) and there are epochs to share out.
+inline int slices_for(int64_t n, int N) {
+    return n < 4 * 608 * 128 && N >= 16 ? 4 : 1;
 }
 
 // FP64 ln L of one sample with the star's epochs read from global memory, in

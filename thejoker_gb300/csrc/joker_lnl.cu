@@ -36,47 +36,27 @@ namespace joker {
 // it does not take runs in doubles (fp64_lnl_doubles).  In doubles the FP64
 // pipe bounded it (70-90 FP64 instructions per epoch, 16 cycles of an SM
 // each); in fixed point instruction issue does.  2^20 samples x 16 epochs:
-// 2267 us in doubles, 373 us; 1.5e6 x 40 with the jitter: 9041, 1484 us.
+// 2267 us in doubles, 352 us; 1.5e6 x 40 with the jitter: 9041, 1520 us.
 template <int L, bool JIT>
-__global__ void __launch_bounds__(128)
-lnl_fp64_kernel(LnlArgs a) {
-    __shared__ fx::EpochFx sm[TILE];
-    __shared__ int s_item;
-    int staged_star = -1;
-    for (;;) {
-        __syncthreads();
-        if (threadIdx.x == 0) s_item = atomicAdd(a.queue, 1);
-        __syncthreads();
-        const int it = s_item;
-        if (it >= item_count(a)) break;
+__global__ void __launch_bounds__(SLICED_BLOCK)
+lnl_fp64_kernel(LnlArgs a, int S) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int per = SLICED_BLOCK / S;                     // samples per pass
+    const int mine = (threadIdx.x >> 5) / S * 32 + (threadIdx.x & 31);
+    const int n_items = item_count(a);
+    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
         const WorkItem w = get_item(a, it);
         const StarRec &st = a.stars[w.star];
-        const int N = st.n_epochs;
-        const bool single = N <= TILE;
-        if (single && w.star != staged_star) {
-            stage_epochs_fx(sm, a.ep64 + (size_t)st.epoch_off * REC64, N);
-            staged_star = w.star;
-            __syncthreads();
-        }
         unsigned long long *mk = a.max_key ? a.max_key + w.max_slot : nullptr;
-        for (int base = 0; base < w.count; base += blockDim.x) {
-            const int j = base + threadIdx.x;
+        for (int base = 0; base < w.count; base += per) {
+            const int j = base + mine;
             const bool active = j < w.count;
             const int64_t row = (w.row0 + (active ? j : 0)) * a.stride;
             const double P = a.P[row], e = a.e[row], om = a.om[row], M0 = a.M0[row];
             const double s = JIT ? a.s[row] : 0.0;
             AccFx<L, JIT> acc;
             bool ok = acc.init(st, P, e, om, M0, s);
-            for (int t0 = 0; t0 < N; t0 += TILE) {
-                const int nt = min(TILE, N - t0);
-                if (!single) {
-                    __syncthreads();
-                    stage_epochs_fx(sm, a.ep64 + ((size_t)st.epoch_off + t0) * REC64, nt);
-                    __syncthreads();
-                }
-                if (active && ok)
-                    for (int i = 0; i < nt; ++i) acc.add(sm[i]);
-            }
+            if (!sliced_epochs(acc, active && ok, st, a.ep64, smem, S)) continue;
             double lnl = 0.0;
             if (active) {
                 ok = ok && !acc.orb.bad;
@@ -114,10 +94,34 @@ __global__ void prepare_cache_kernel(const double *__restrict__ chunk, int64_t n
 cudaError_t launch_lnl_packed(int precision, int L, bool jit, const LnlArgs &a, int block,
                               cudaStream_t st);
 
+// One block per work item (blocks start in order as others end, which spreads
+// uneven items as a work counter would, without the launch that zeroes one);
+// a count in device memory is shared out over a grid of one wave.
+template <int L, bool JIT>
+static cudaError_t launch_fp64_LJ(LnlArgs a, cudaStream_t st) {
+    int grid = a.n_items, S = 1;
+    if (a.n_items_dev) {
+        const cudaError_t e = persistent_grid(
+            reinterpret_cast<const void *>(lnl_fp64_kernel<L, JIT>), SLICED_BLOCK, &grid);
+        if (e != cudaSuccess) return e;
+    } else if (!a.items) {
+        S = slices_for(a.count * a.n_sel, a.max_epochs);
+        const int64_t chunk = SLICED_BLOCK / S, ips = (a.count + chunk - 1) / chunk;
+        if (ips * a.n_sel <= INT32_MAX) {
+            a.chunk = (int)chunk;
+            a.ips = ips;
+            grid = a.n_items = (int)(ips * a.n_sel);
+        }
+    }
+    if (grid < 1) return cudaSuccess;
+    lnl_fp64_kernel<L, JIT><<<grid, SLICED_BLOCK, sliced_smem<L, JIT>(S), st>>>(a, S);
+    count_launch();
+    return cudaGetLastError();
+}
+
 template <int L>
-static cudaError_t launch_fp64_L(bool jit, const LnlArgs &a, int block, cudaStream_t st) {
-    if (jit) return launch_persistent(lnl_fp64_kernel<L, true>, a, block, st);
-    return launch_persistent(lnl_fp64_kernel<L, false>, a, block, st);
+static cudaError_t launch_fp64_L(bool jit, const LnlArgs &a, cudaStream_t st) {
+    return jit ? launch_fp64_LJ<L, true>(a, st) : launch_fp64_LJ<L, false>(a, st);
 }
 
 template <int L, int VAR>
@@ -153,12 +157,12 @@ cudaError_t launch_lnl(int precision, int L, bool jit, const LnlArgs &a, int blo
     }
     if (precision == JOKER_FP64) {
         switch (L) {
-            case 1: return launch_fp64_L<1>(jit, a, block, st);
-            case 2: return launch_fp64_L<2>(jit, a, block, st);
-            case 3: return launch_fp64_L<3>(jit, a, block, st);
-            case 4: return launch_fp64_L<4>(jit, a, block, st);
-            case 5: return launch_fp64_L<5>(jit, a, block, st);
-            case 6: return launch_fp64_L<6>(jit, a, block, st);
+            case 1: return launch_fp64_L<1>(jit, a, st);
+            case 2: return launch_fp64_L<2>(jit, a, st);
+            case 3: return launch_fp64_L<3>(jit, a, st);
+            case 4: return launch_fp64_L<4>(jit, a, st);
+            case 5: return launch_fp64_L<5>(jit, a, st);
+            case 6: return launch_fp64_L<6>(jit, a, st);
         }
     } else if (a.mx_a == nullptr) {
         return launch_lnl_packed(precision, L, jit, a, block, st);

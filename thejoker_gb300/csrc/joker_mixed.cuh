@@ -17,14 +17,6 @@ __device__ __forceinline__ void stage_epochs(T *sm, const T *src, int n) {
     for (int i = threadIdx.x; i < nvec; i += blockDim.x) d4[i] = __ldg(s4 + i);
 }
 
-// The fixed-point halves of n FP64 epoch records.
-__device__ __forceinline__ void stage_epochs_fx(fx::EpochFx *sm, const double *src, int n) {
-    const int4 *s4 = reinterpret_cast<const int4 *>(src + FX64);
-    int4 *d4 = reinterpret_cast<int4 *>(sm);
-    for (int i = threadIdx.x; i < n * 4; i += blockDim.x)
-        d4[i] = __ldg(s4 + (i >> 2) * (REC64 / 2) + (i & 3));
-}
-
 // Warp-aggregated raise of a running maximum.
 __device__ __forceinline__ void warp_max_update(unsigned long long *key, unsigned long long k) {
 #pragma unroll

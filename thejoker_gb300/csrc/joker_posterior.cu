@@ -1,5 +1,4 @@
-// Per-sample FP64 work after the acceptance pass, one warp per sample (lanes
-// over epochs):
+// Per-sample FP64 work after the acceptance pass:
 //
 // * the Gaussian posterior of the linear parameters of accepted samples --
 //   the a and Ainv that CJokerHelper.likelihood_worker(1) builds
@@ -13,7 +12,200 @@
 
 namespace joker {
 
-// Posterior of the linear parameters of one sample.  With W = diag(w),
+// log of a product of positive doubles: exponents as integers, mantissas
+// multiplied, one logarithm for all; what has no normal exponent (zero,
+// subnormal, inf, NaN, negative) through log by itself.
+struct LogProd {
+    double m = 1.0, rest = 0.0;
+    int e = 0;
+    __device__ __forceinline__ void times(double x) {
+        const int hi = __double2hiint(x), ex = hi >> 20;
+        if (ex <= 0 || ex >= 2047) { rest += log(x); return; }
+        e += ex - 1023;
+        m *= __hiloint2double((hi & 0x000fffff) | 0x3ff00000, __double2loint(x));
+    }
+    __device__ __forceinline__ double value() const {
+        return rest + fma((double)e, 0.69314718055994530942, log(m));
+    }
+};
+
+// Posterior of the linear parameters of one sample from G0 = M W M^T (lower
+// triangle), q = M W (y - M^T mu) and rWr: with G = Lambda^-1 + G0,
+// a = mu + G^-1 q, A = G^-1 (G = Lw D Lw^T, A = Lw^-T D^-1 Lw^-1), and ln L
+// from the same factorisation.  lp holds the factors of the log determinant
+// that are known beforehand, logdet0 the rest of it.
+template <int L>
+__device__ __forceinline__ void posterior_tail(const StarRec &st, double (&G)[L][L],
+                                               const double (&q)[L], double rWr, double logdet0,
+                                               LogProd lp, double lam0, double *a_out,
+                                               double *A_out, double *lnl_out) {
+    double ilam0 = st.ilam[0];
+    if (st.k_scaled) ilam0 = lam0 < 1e300 ? rcp_newton(lam0) : 1.0 / lam0;
+    lp.times(lam0);
+    double rD[L], Lw[L][L];
+    bool ok = true;
+    {
+        double D[L];
+#pragma unroll
+        for (int k = 0; k < L; ++k) {
+            double dk = G[k][k] + (k == 0 ? ilam0 : st.ilam[k]);
+#pragma unroll
+            for (int m = 0; m < k; ++m) dk -= Lw[k][m] * Lw[k][m] * D[m];
+            D[k] = dk;
+            ok = ok && dk > 0.0;
+            lp.times(dk);
+            rD[k] = dk < 1e300 ? rcp_newton(dk) : 1.0 / dk;
+#pragma unroll
+            for (int i = k + 1; i < L; ++i) {
+                double v = G[i][k];
+#pragma unroll
+                for (int m = 0; m < k; ++m) v -= Lw[i][m] * Lw[k][m] * D[m];
+                Lw[i][k] = v * rD[k];
+            }
+        }
+    }
+    // z = Lw^-1 q, quad = z^T D^-1 z, x = Lw^-T D^-1 z
+    double x[L], quad = 0.0;
+#pragma unroll
+    for (int k = 0; k < L; ++k) {
+        double v = q[k];
+#pragma unroll
+        for (int m = 0; m < k; ++m) v -= Lw[k][m] * x[m];
+        x[k] = v;
+        quad = fma(v * v, rD[k], quad);
+    }
+#pragma unroll
+    for (int k = L - 1; k >= 0; --k) {
+        double v = x[k] * rD[k];
+#pragma unroll
+        for (int m = k + 1; m < L; ++m) v -= Lw[m][k] * x[m];
+        x[k] = v;
+    }
+#pragma unroll
+    for (int k = 0; k < L; ++k) a_out[k] = ok ? st.mu[k] + x[k] : NAN;
+    // Lw <- Lw^-1 (unit lower triangle), column by column
+#pragma unroll
+    for (int c = 0; c < L; ++c)
+#pragma unroll
+        for (int i = c + 1; i < L; ++i) {
+            double v = Lw[i][c];
+#pragma unroll
+            for (int m = c + 1; m < i; ++m) v = fma(Lw[i][m], Lw[m][c], v);
+            Lw[i][c] = -v;
+        }
+#pragma unroll
+    for (int i = 0; i < L; ++i)
+#pragma unroll
+        for (int c = 0; c <= i; ++c) {
+            double v = i == c ? rD[i] : rD[i] * Lw[i][c];
+#pragma unroll
+            for (int k = i + 1; k < L; ++k) v = fma(Lw[k][i] * rD[k], Lw[k][c], v);
+            A_out[i * L + c] = A_out[c * L + i] = ok ? v : NAN;
+        }
+    if (lnl_out) *lnl_out = ok ? -0.5 * (rWr - quad + logdet0 + lp.value()) : INFINITY;
+}
+
+// The same without jitter, where only K's row A00, A0, b0 of the system depends
+// on the sample: with the star's own C^-1 and beta = C^-1 c (trend block),
+// v = C^-1 A0 and the Schur complement s = A00 + 1/Lambda0 - A0 v,
+//   K = (b0 - A0 beta) / s,  trend = mu + beta - v K,
+//   A = [1/s, -v^T/s; -v/s, C^-1 + v v^T / s]
+// (mu0 = 0).  Eliminating the full system per sample instead would lose what
+// the trend explains of y' (ln L: 1e-9 .. 1e-11 relative with a trend).
+template <int L>
+__device__ __forceinline__ void posterior_schur(const StarRec &st, double A00, const double *A0,
+                                                double b0, double lam0, double *a_out,
+                                                double *A_out, double *lnl_out) {
+    double v[MAXL], gv = 0.0, u = b0;
+#pragma unroll
+    for (int j = 1; j < L; ++j) {
+        v[j] = 0.0;
+#pragma unroll
+        for (int k = 1; k < L; ++k) v[j] = fma(st.Cinv[j * MAXL + k], A0[k], v[j]);
+        gv = fma(A0[j], v[j], gv);
+        u = fma(-A0[j], st.cC[j], u);
+    }
+    const double ls = fma(lam0, A00 - gv, 1.0);               // Lambda0 s
+    const bool ok = ls > 0.0;
+    const double is = lam0 * (ls < 1e300 ? rcp_newton(ls) : 1.0 / ls);
+    const double K = u * is;
+    a_out[0] = ok ? K : NAN;
+    A_out[0] = ok ? is : NAN;
+#pragma unroll
+    for (int j = 1; j < L; ++j) {
+        const double w = v[j] * is;
+        a_out[j] = ok ? st.mu[j] + fma(-v[j], K, st.cC[j]) : NAN;
+        A_out[j] = A_out[j * L] = ok ? -w : NAN;
+#pragma unroll
+        for (int k = 1; k <= j; ++k)
+            A_out[j * L + k] = A_out[k * L + j] = ok ? fma(w, v[k], st.Cinv[j * MAXL + k]) : NAN;
+    }
+    if (lnl_out)
+        *lnl_out = ok ? -0.5 * (fma(-u, K, st.chi2_0) + st.logdet_const + log(ls)) : INFINITY;
+}
+
+// In doubles, one thread: the form for what the fixed-point one does not take.
+template <int L>
+__device__ __noinline__ void posterior_doubles(const StarRec &st, const double *ep64, double P,
+                                               double e, double om, double M0, double s, int k_clip,
+                                               double *a_out, double *A_out, double *lnl_out) {
+    Acc64<L, true> acc;
+    acc.init(st, P, e, om, M0, s);
+    const double *rec = ep64 + (size_t)st.epoch_off * REC64;
+    for (int i = 0; i < st.n_epochs; ++i, rec += REC64) {
+        double T[MAXL];
+#pragma unroll
+        for (int k = 1; k < L; ++k) T[k - 1] = __ldg(rec + 2 + k);
+        acc.add(__ldg(rec), __ldg(rec + 1), __ldg(rec + 2), T);
+    }
+    posterior_tail<L>(st, acc.G, acc.q, acc.rWr, st.log_norm_rest - acc.sum_log_w(st), LogProd(),
+                      k_prior_variance(st, P, e, k_clip != 0), a_out, A_out, lnl_out);
+}
+
+// One sample per thread, epochs shared out over S warps (sliced_epochs).
+// A warp per sample in doubles spent its time
+// on idle lanes -- 40 epochs on 64 lanes, ten FP64 shuffles a sum, the tail on
+// one lane: 100003 rows x 40 epochs, three linear parameters took
+// 4326 us, now 105.
+template <int L, bool JIT>
+__global__ void __launch_bounds__(SLICED_BLOCK)
+posterior_kernel(const StarRec *stars, const double *ep64, int star, const double *P,
+                 const double *E, const double *OM, const double *M0, const double *S,
+                 int64_t stride, const int64_t *rows, int64_t n, int k_clip, double *a, double *A,
+                 double *lnl, int slices) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const StarRec &st = stars[star];
+    const int64_t i = blockIdx.x * (int64_t)(SLICED_BLOCK / slices) +
+                      (threadIdx.x >> 5) / slices * 32 + (threadIdx.x & 31);
+    const bool active = i < n;
+    const int64_t r = rows[active ? i : n - 1] * stride;
+    const double p = P[r], e = E[r], om = OM[r], m0 = M0[r], s = JIT ? S[r] : 0.0;
+    AccFx<L, JIT> acc;
+    bool ok = acc.init(st, p, e, om, m0, s);
+    if (!sliced_epochs(acc, active && ok, st, ep64, smem, slices) || !active) return;
+    double *a_out = a + i * L, *A_out = A + i * L * L, *l_out = lnl ? lnl + i : nullptr;
+    if (!ok || acc.orb.bad) {
+        posterior_doubles<L>(st, ep64, p, e, om, m0, s, k_clip, a_out, A_out, l_out);
+        return;
+    }
+    const double lam0 = k_prior_variance(st, p, e, k_clip != 0);
+    if constexpr (JIT) {
+        double G[L][L], q[L], rWr, f;
+        LogProd lp;
+        acc.system(st, G, q, rWr);
+        const double lr = acc.log_rest(st, f);
+        lp.times(f);
+        posterior_tail<L>(st, G, q, rWr, st.log_norm_rest - st.sum_log_ivar + lr, lp, lam0, a_out,
+                          A_out, l_out);
+    } else {
+        double A00, b0, A0[MAXL];
+        acc.k_row(st, A00, b0, A0);
+        posterior_schur<L>(st, A00, A0, b0, lam0, a_out, A_out, l_out);
+    }
+}
+
+// For a star without a fixed-point form, one warp per sample, lanes over
+// epochs.  Posterior of the linear parameters of one sample.  With W = diag(w),
 // G = Lambda^-1 + M W M^T and q = M W (y - M^T mu) (Acc64 with the jitter
 // form), a = mu + G^-1 q, A = G^-1, and ln L from the same factorisation.
 template <int L>
@@ -103,7 +295,7 @@ __device__ __noinline__ void posterior_one(const StarRec &st, const double *ep64
 }
 
 template <int L>
-__global__ void __launch_bounds__(256) posterior_kernel(const StarRec *stars, const double *ep64,
+__global__ void __launch_bounds__(256) posterior_warp_kernel(const StarRec *stars, const double *ep64,
                                                         int star, const double *P, const double *E,
                                                         const double *OM, const double *M0,
                                                         const double *S, int64_t stride,
@@ -185,29 +377,52 @@ cudaError_t launch_rv_elements(const double *t, int n_t, const double *el, int64
     return cudaGetLastError();
 }
 
+template <int L, bool JIT>
+static cudaError_t launch_posterior_LJ(const StarRec *stars, const double *ep64, int star,
+                                       int max_epochs, const double *P, const double *E,
+                                       const double *OM, const double *M0, const double *S,
+                                       int64_t stride, const int64_t *rows, int64_t n, int k_clip,
+                                       double *a, double *A, double *lnl, cudaStream_t st) {
+    const int sl = slices_for(n, max_epochs), per = SLICED_BLOCK / sl;
+    const int64_t blocks = (n + per - 1) / per;
+    if (blocks > INT32_MAX) return cudaErrorInvalidValue;
+    posterior_kernel<L, JIT><<<(unsigned)blocks, SLICED_BLOCK, sliced_smem<L, JIT>(sl), st>>>(
+        stars, ep64, star, P, E, OM, M0, S, stride, rows, n, k_clip, a, A, lnl, sl);
+    count_launch();
+    return cudaGetLastError();
+}
+
+// fixed: the star has a fixed-point form (stars_fixed).
 template <int L>
 static cudaError_t launch_posterior_L(const StarRec *stars, const double *ep64, int star,
-                                      const double *P, const double *E, const double *OM,
-                                      const double *M0, const double *S, int64_t stride,
-                                      const int64_t *rows, int64_t n, int jit, int k_clip,
-                                      double *a, double *A, double *lnl, cudaStream_t st) {
+                                      bool fixed, int max_epochs, const double *P,
+                                      const double *E, const double *OM, const double *M0,
+                                      const double *S, int64_t stride, const int64_t *rows,
+                                      int64_t n, int jit, int k_clip, double *a, double *A,
+                                      double *lnl, cudaStream_t st) {
+    if (fixed && jit)
+        return launch_posterior_LJ<L, true>(stars, ep64, star, max_epochs, P, E, OM, M0, S, stride,
+                                            rows, n, k_clip, a, A, lnl, st);
+    if (fixed)
+        return launch_posterior_LJ<L, false>(stars, ep64, star, max_epochs, P, E, OM, M0, S, stride,
+                                             rows, n, k_clip, a, A, lnl, st);
     const int64_t warps = n < 152 * 8 * 4 ? n : 152 * 8 * 4;
     const unsigned grid = (unsigned)((warps + 7) / 8);
-    posterior_kernel<L><<<grid, 256, 0, st>>>(stars, ep64, star, P, E, OM, M0, S, stride, rows,
-                                              n, jit, k_clip, a, A, lnl);
+    posterior_warp_kernel<L><<<grid, 256, 0, st>>>(stars, ep64, star, P, E, OM, M0, S, stride, rows,
+                                                   n, jit, k_clip, a, A, lnl);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_posterior(int L, const StarRec *stars, const double *ep64, int star,
-                             const double *P, const double *E, const double *OM,
+                             bool fixed, int max_epochs, const double *P, const double *E, const double *OM,
                              const double *M0, const double *S, int64_t stride,
                              const int64_t *rows, int64_t n, int jit, int k_clip, double *a,
                              double *A, double *lnl, cudaStream_t st) {
     switch (L) {
 #define JOKER_POST_CASE(LL) \
-        case LL: return launch_posterior_L<LL>(stars, ep64, star, P, E, OM, M0, S, stride, rows, \
-                                               n, jit, k_clip, a, A, lnl, st);
+        case LL: return launch_posterior_L<LL>(stars, ep64, star, fixed, max_epochs, P, E, OM, M0, S, \
+                                               stride, rows, n, jit, k_clip, a, A, lnl, st);
         JOKER_POST_CASE(1) JOKER_POST_CASE(2) JOKER_POST_CASE(3)
         JOKER_POST_CASE(4) JOKER_POST_CASE(5) JOKER_POST_CASE(6)
 #undef JOKER_POST_CASE
@@ -232,6 +447,8 @@ namespace joker {
 void set_last_error(const char *msg);
 void stars_internals(const joker_stars *s, const StarRec **recs, const double **ep64,
                      const float **ep32, int *n_stars, int *L, int *jit, int **queue);
+int stars_max_epochs(const joker_stars *s);
+bool stars_fixed(const joker_stars *s, int star);
 void cache_internals(const joker_cache *c, int64_t *cap, const double **P, const double **E,
                      const double **OM, const double **M0, const double **S, int64_t *stride,
                      const float4 **mx_a, const float4 **mx_b, const float **mx_s2);
@@ -258,7 +475,8 @@ extern "C" int joker_linear_posterior(const joker_stars *stars, const joker_cach
         return post_fail(JOKER_EINVAL, "joker_linear_posterior: star out of range");
     int64_t cap, stride; const double *P, *E, *OM, *M0, *S; const float4 *ma, *mb; const float *ms;
     cache_internals(cache, &cap, &P, &E, &OM, &M0, &S, &stride, &ma, &mb, &ms);
-    const cudaError_t e = launch_posterior(L, recs, ep64, star, P, E, OM, M0, S, stride, d_rows,
+    const cudaError_t e = launch_posterior(L, recs, ep64, star, stars_fixed(stars, star),
+                                           stars_max_epochs(stars), P, E, OM, M0, S, stride, d_rows,
                                            n, jit, k_clip, d_a, d_A, d_lnl, (cudaStream_t)stream);
     if (e != cudaSuccess) return post_fail(JOKER_ECUDA, cudaGetErrorString(e));
     return JOKER_OK;
