@@ -81,3 +81,22 @@ def test_prior_mean(cuda):
         chunk = synth_chunk(rng, 64, jitter=jitter)
         chunk[:, 1] = np.minimum(chunk[:, 1], 0.9)
         _check(star, chunk, jitter)
+
+
+@pytest.mark.parametrize("rows,times", [(1, 1), (3, 7), (2, 255), (5, 256), (33, 257), (2, 1001)])
+def test_rv_curves(cuda, rows, times):
+    """Curves that end inside, at and beyond a warp's share of times, times on
+    both sides of t0, and one orbit beyond the fixed-point form."""
+    from thejoker_gb300 import device as dev
+    from thejoker_gb300.linear import rv_unit_columns
+    rng = np.random.default_rng(rows * 10000 + times)
+    c = synth_chunk(rng, rows)
+    c[:, 1] = np.minimum(c[:, 1], 0.9)
+    c[-1, 1] = 0.9995
+    K = rng.uniform(1.0, 50.0, rows)
+    t, t0 = 2456000.0 + rng.uniform(0.0, 2000.0, times), 2456700.0
+    el = np.stack([c[:, 0], K, c[:, 1], c[:, 2], c[:, 3]], 1)
+    got = dev.rv_from_elements(torch.from_numpy(t).cuda(), torch.from_numpy(el).cuda(), t0)
+    want = K[:, None] * rv_unit_columns(t, t0, c[:, 0], c[:, 1], c[:, 2], c[:, 3])
+    tol = 1e-9 * K / (1.0 - c[:, 1]) ** 2
+    assert np.all(np.abs(got.cpu().numpy() - want) <= tol[:, None])

@@ -185,6 +185,15 @@ JOKER_FX int64_t fixed62(double x) {
     return clamp62((int64_t)shift((b & 0xfffffffffffffull) | 0x10000000000000ull,
                                   (int)(b >> 52) - 1013));
 }
+// x 2^q, the bits below the unit dropped, for |x| 2^q < 2^63
+JOKER_FX int64_t fixed_signed(double x, int q) {
+    const uint64_t b = bits_of(x);
+    const int be = (int)(b >> 52) & 0x7ff;
+    if (be == 0) return 0;
+    const int64_t v = (int64_t)shift((b & 0xfffffffffffffull) | 0x10000000000000ull,
+                                     be - 1075 + q);
+    return (b >> 63) ? -v : v;
+}
 // a (radians, |a| < 2^10) in turns mod 1, Q64
 JOKER_FX uint64_t turns64(double a) {
     const uint64_t b = bits_of(a);
