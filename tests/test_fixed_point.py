@@ -24,7 +24,7 @@ extern "C" int column(int tsh, int64_t t0, double P, double e, double om, double
     Orbit o;
     if (!o.init(tsh, t0, P, e, om, M0)) return 0;
     *m = o.column(t);
-    return o.bad ? -1 : 1;
+    return o.bad() ? -1 : 1;
 }
 extern "C" int64_t quotient(int64_t num, int64_t den) { return div61(num, den); }
 extern "C" int64_t root(int64_t y) { return sqrt62(y); }

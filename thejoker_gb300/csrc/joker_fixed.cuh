@@ -63,16 +63,17 @@ JOKER_FX trig_entry trig_node(int k) {
     return kTrig[k];
 #endif
 }
-// a b 2^-62 to 2 units (truncated): Qi x Qj -> Q(i + j - 62)
-JOKER_FX int64_t mul(limbs a, limbs b) {
-    return wide(a.h, b.h) + ((wide(a.h, b.l) + wide(a.l, b.h)) >> 31);
-}
 JOKER_FX int32_t hi32(int32_t a, int32_t b) {
 #ifdef __CUDA_ARCH__
     return __mulhi(a, b);
 #else
     return (int32_t)(wide(a, b) >> 32);
 #endif
+}
+// a b 2^-62 to 5 units (truncated): Qi x Qj -> Q(i + j - 62).  The sum of the
+// two high halves stays in 32 bits: each is below 2^30 in size.
+JOKER_FX int64_t mul(limbs a, limbs b) {
+    return wide(a.h, b.h) + 2 * (int64_t)(hi32(a.h, b.l) + hi32(a.l, b.h));
 }
 // u v, with u v's 64 bits: the three partial products above 2^32 of the four
 JOKER_FX uint64_t hi64(uint64_t u, uint64_t v) {
@@ -89,6 +90,8 @@ JOKER_FX float lg2_a(float x) { float r; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"
 JOKER_FX float ex2_a(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 JOKER_FX int32_t rint_a(float x) { return __float2int_rn(x); }   // saturates, NaN -> 0
 JOKER_FX float fma_a(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+JOKER_FX float max_a(float a, float b) { return fmaxf(a, b); }
+JOKER_FX int32_t max_a(int32_t a, int32_t b) { return max(a, b); }
 #else
 JOKER_FX int clz64(uint64_t v) { return v ? __builtin_clzll(v) : 64; }
 JOKER_FX float rcp_a(float x) { return 1.0f / x; }
@@ -102,6 +105,8 @@ JOKER_FX int32_t rint_a(float x) {
     return (int32_t)std::nearbyint(x);
 }
 JOKER_FX float fma_a(float a, float b, float c) { return std::fma(a, b, c); }
+JOKER_FX float max_a(float a, float b) { return a < b ? b : a; }
+JOKER_FX int32_t max_a(int32_t a, int32_t b) { return a < b ? b : a; }
 #endif
 
 // num / den in Q61 for 0 < den < 2^62 and |num| <= den (1 + 2^-40), to 16
@@ -131,18 +136,19 @@ JOKER_FX float to_float(int64_t v) {
     return fma_a((float)h, 0x1p32f, (float)l);
 }
 
-// sin and cos (Q61) of a node's angle plus r, r8 = 2^8 r (Q62), |r| < 2^-8.5:
-// the Taylor series of sin r and cos r to r^5, then the addition formulas.
-JOKER_FX void turn_by(trig_entry tab, limbs S, limbs C, int64_t r8, int64_t &s1, int64_t &c1) {
-    const limbs r = split(r8);
-    const int64_t R2 = wide(r.h, r.h) + (wide(r.h, r.l) >> 30);       // 2^16 r^2 (Q62)
-    const int32_t R2h = (int32_t)(R2 >> 30);                          // 2^48 r^2
+// sin and cos (Q61) of a node's angle plus r (Q62), |r| < 2^-8.4: the Taylor
+// series of sin r and cos r to r^5, then the addition formulas.
+JOKER_FX void turn_by(trig_entry tab, limbs S, limbs C, int64_t rq, int64_t &s1, int64_t &c1) {
+    const limbs r = split(rq);
+    const int32_t rh = (int32_t)(rq >> 23);                           // 2^39 r
+    const int64_t R2 = mul(r, r);                                     // r^2 (Q62)
+    const int32_t R2h = (int32_t)(R2 >> 14);                          // 2^48 r^2
     const int32_t R4h = hi32(R2h, R2h);                               // 2^64 r^4
     const int32_t g = hi32(R2h, 715827883) - hi32(R4h, 546);          // 2^48 (r^2/6 - r^4/120)
-    const limbs sr = split(r8 - (wide(r.h, g) >> 17));                // 2^8 sin r (Q62)
-    const limbs nc = split(R2 - (wide(R4h, 5592405) >> 12));          // 2^17 (1 - cos r) (Q62)
-    s1 = tab.s + (mul(sr, C) >> 8) - (mul(nc, S) >> 17);
-    c1 = tab.c - (mul(sr, S) >> 8) - (mul(nc, C) >> 17);
+    const limbs sr = split(rq - (wide(rh, g) >> 25));                 // sin r (Q62)
+    const limbs nc = split((R2 >> 1) - hi32(R4h, 44739243));          // 1 - cos r (Q62)
+    s1 = tab.s + mul(sr, C) - mul(nc, S);
+    c1 = tab.c - mul(sr, S) - mul(nc, C);
 }
 
 // ------------------------------------------------- doubles to fixed point
@@ -234,9 +240,11 @@ struct Orbit {
     limbs A, B;                // cos w, -sin w sqrt(1 - e^2) (Q62)
     int64_t D;                 // e cos w (Q61)
     float ef, omef, a1f;       // e, 1 - e, Markley's a1
+    float ef30;                // e 2^-30
     float cs;                  // 2^(61 - sg): scale of the last correction
     int32_t psg;               // 2^sg
-    int32_t bad;               // an iteration left its range
+    int32_t far_r;             // the largest |ri| and |dl| of the columns so far
+    float far_d;
 
     // Integer times are t = dt 2^tsh - t0.  False: outside the fixed-point
     // form's range, whose lines are the phase's 2^32 turns per time scale,
@@ -244,7 +252,8 @@ struct Orbit {
     // least as exact as the FP64 one (its last FP32 correction grows as
     // 1 / f'^2 beyond).
     JOKER_FX bool init(int tsh, int64_t t0, double P, double e_, double om, double M0) {
-        bad = 0;
+        far_r = 0;
+        far_d = 0.0f;
         const uint64_t pb = bits_of(P);
         const int pe = (int)(pb >> 52);                       // sign bit too
         const int s = 1088 - tsh - pe;
@@ -264,20 +273,21 @@ struct Orbit {
         e = split(e62);
         ep = split((int64_t)hi64((uint64_t)e62 << 2, INV_2PI_Q64));
         ef = to_float(e62) * 0x1p-62f;
+        ef30 = ef * 0x1p-30f;
         omef = to_float(ONE62 - e62) * 0x1p-62f;
         a1f = 1.6f * 3.14159265358979f / (9.8696044011f - 6.0f) * rcp_a(1.0f + ef);
         const int sg = 5 + 126 - (int)(float_bits(omef) >> 23);
         cs = float_of((uint32_t)(127 + 61 - sg) << 23);
         psg = 1 << sg;
-        // omega: the node nearest to |turn| and the rest of the angle
+        // omega: the node nearest to |turn| and the rest of the angle, r = 2 pi 2^-64 rest
         const uint64_t w = turns64(om);
         const bool neg = (int64_t)w < 0;
         const uint64_t aw = neg ? 0 - w : w;                   // [0, 2^63]
         const int k = (int)((aw + (1ull << 52)) >> 53);        // 0..1024
         const trig_entry tab = trig_node(k);
-        const int64_t rho = (int64_t)(aw - ((uint64_t)k << 53)) << 9;
+        const int64_t rho = (int64_t)(aw - ((uint64_t)k << 53)) << 9;   // r = rho 2^-62 pi/4 2^-8
         int64_t sw, cw;
-        turn_by(tab, split(tab.s), split(tab.c), mul(split(rho), split(PI_4_Q62)), sw, cw);
+        turn_by(tab, split(tab.s), split(tab.c), mul(split(rho), split(PI_4_Q62)) >> 8, sw, cw);
         D = mul(e, split(cw));
         A = split(twice(cw));
         const int64_t om2 = ONE62 - mul(e, e);
@@ -285,12 +295,13 @@ struct Orbit {
         B = split(twice(neg ? b : -b));
         return true;
     }
-    // The column m = cos(w + f) + e cos w (Q61) at integer time t.
+    // The column m = cos(w + f) + e cos(w) (Q61) at integer time t.
     JOKER_FX int64_t column(uint64_t t) {
-        // phase in turns mod 1, Q64, and its size in [0, 1/2]
+        // phase in turns mod 1, Q64; its sign and its size in [0, 1/2] (to a
+        // unit: the complement stands for the negative)
         const uint64_t turn = ph0 + t * Ri + hi64(t, Rf);
-        const bool neg = (int64_t)turn < 0;
-        const uint64_t x = neg ? 0 - turn : turn;
+        const int64_t sgn = (int64_t)turn >> 63;
+        const uint64_t x = turn ^ (uint64_t)sgn;
         const int64_t x63 = (int64_t)(x >> 1);
         const float xf = fma_a((float)(uint32_t)(x >> 32), TWO_PI_FX * 0x1p-32f,
                                (float)(uint32_t)x * (TWO_PI_FX * 0x1p-64f));
@@ -300,46 +311,44 @@ struct Orbit {
         const float d = fma_a(alpha, ef, 3.0f * omef);
         const float x2 = xf * xf;
         const float ad = alpha * d;
-        const float q = fma_a(2.0f * ad, omef, -x2);
-        const float r = xf * fma_a(3.0f * ad, d - omef, x2);
+        const float q = fma_a(ad, 2.0f * omef, -x2);
+        const float r = xf * fma_a(ad, fma_a(3.0f, d, -3.0f * omef), x2);
         const float qq = q * q;
-        const float disc = fma_a(qq, q, r * r);
-        const float sq = disc > 0.0f ? disc * rsqrt_a(disc) : 0.0f;
-        const float w = ex2_a(0.6666667f * lg2_a(r + sq));
+        const float disc = max_a(fma_a(qq, q, r * r), 1e-30f);
+        const float w = ex2_a(0.6666667f * lg2_a(fma_a(disc, rsqrt_a(disc), r)));
         const float den3 = fma_a(w, w + q, qq);
         const float E0 = fma_a(xf, den3, 2.0f * r * w) * rcp_a(den3 * d);
         int32_t i0 = rint_a(E0 * (0x1p32f / TWO_PI_FX));
-        // node k of the table (2048 a turn) nearest to it
         i0 = i0 < 0 ? 0 : i0;
+        // node k of the table (2048 a turn) nearest to it
         const int k = (int)(((uint32_t)i0 + (1u << 20)) >> 21);          // 0..1024
         const trig_entry tab = trig_node(k);
         const limbs S = split(tab.s), C = split(tab.c);                   // Q61
-        const float Sf = (float)S.h * 0x1p-30f, Cf = (float)C.h * 0x1p-30f;
+        const float Sf = (float)S.h, Cf = (float)C.h;                     // 2^30 sin, cos
         int32_t ri = (int32_t)((uint32_t)i0 - ((uint32_t)k << 21));       // Q32 turns
         // first step: f(E0) to 2^-34 turns, Halley's correction in FP32
-        float rf = (float)ri * (TWO_PI_FX * 0x1p-32f);
+        const float rf = (float)ri * (TWO_PI_FX * 0x1p-32f);
         const float hr2 = 0.5f * rf * rf;
         const float srf = fma_a(rf * hr2, -1.0f / 3.0f, rf);
-        const float ds0 = fma_a(Cf, srf, -Sf * hr2);                      // sin E0 - S
+        const float ds0 = fma_a(Cf, srf, -Sf * hr2);                      // 2^30 (sin E0 - S)
         const float c0 = fma_a(-Sf, srf, fma_a(-Cf, hr2, Cf));
         const int64_t f0i = ((int64_t)i0 << 31) - x63 - wide(ep.h, S.h);  // Q63
-        const float f0 = fma_a((float)(int32_t)(f0i >> 21), TWO_PI_FX * 0x1p-42f, -ef * ds0);
-        const float f2 = ef * (Sf + ds0);
-        const float f1 = fma_a(-ef, c0, 1.0f);
+        const float f0 = fma_a((float)(int32_t)(f0i >> 21), TWO_PI_FX * 0x1p-42f, -ef30 * ds0);
+        const float f2 = ef30 * (Sf + ds0);
+        const float f1 = fma_a(-ef30, c0, 1.0f);
         const float dl0 = f0 * f1 * rcp_a(fma_a(f1, f1, -0.5f * f0 * f2));   // -delta
         ri -= rint_a(dl0 * (0x1p32f / TWO_PI_FX));
-        bad |= (ri > RI_MAX) | (ri < -RI_MAX);
-        // sin E1, cos E1 (Q61) from the node and r = 2 pi ri 2^-32: r8 = 2^8 r (Q62)
+        far_r = max_a(far_r, ri < 0 ? -ri : ri);
+        // sin E1, cos E1 (Q61) from the node and r = 2 pi ri 2^-32 (Q62)
         const int32_t rho = (int32_t)((uint32_t)ri << 10);
-        const int64_t r8 = wide(rho, PI_4_H) + (wide(rho, PI_4_L) >> 31);
         int64_t s1, c1;
-        turn_by(tab, S, C, r8, s1, c1);
+        turn_by(tab, S, C, (wide(rho, PI_4_H) >> 8) + (hi32(rho, PI_4_L) >> 7), s1, c1);
         // last step: f(E1) (Q63 turns) in fixed point, the correction in FP32
         const limbs s1l = split(s1);
         const int64_t E1 = ((int64_t)k << 52) + ((int64_t)ri << 31);
         const float u0 = to_float(E1 - x63 - mul(ep, s1l)) * (TWO_PI_FX * 0x1p-63f);
-        const uint64_t omc = (uint64_t)(ONE61 - c1);
-        const float omcf = fma_a((float)(uint32_t)(omc >> 32), 0x1p-29f,
+        const int64_t omc = ONE61 - c1;
+        const float omcf = fma_a((float)(int32_t)(omc >> 32), 0x1p-29f,
                                  (float)(uint32_t)omc * 0x1p-61f);
         const float i1 = rcp_a(fma_a(ef, omcf, omef));
         const float s1f = (float)s1l.h * 0x1p-30f, c1f = 1.0f - omcf;
@@ -348,14 +357,16 @@ struct Orbit {
         const float hd2 = -0.5f * dl * dl;
         const float dsf = fma_a(c1f, dl, hd2 * s1f) * cs;
         const float dcf = fma_a(-s1f, dl, hd2 * c1f) * cs;
-        bad |= !(fabsf(dl) * cs < 0x1p30f);
-        const int64_t sE0 = s1 + wide(rint_a(dsf), psg);
+        far_d = max_a(far_d, fabsf(dl));
         const limbs cE = split(c1 + wide(rint_a(dcf), psg));
-        const limbs sE = split(neg ? -sE0 : sE0);
+        const limbs sE = split(s1 + wide(rint_a(dsf), psg));
         // (A cos E + B sin E - D) / (1 - e cos E) + D
-        const int64_t num = mul(A, cE) + mul(B, sE) - D;
+        const int64_t num = mul(A, cE) + (mul(B, sE) ^ sgn) - D;
         return div61(num, ONE61 - mul(e, cE)) + D;
     }
+
+    // Whether an iteration left its range in a column so far.
+    JOKER_FX bool bad() const { return far_r > RI_MAX || !(far_d * cs < 0x1p30f); }
 };
 
 // A signed 96-bit sum of 64-bit terms.

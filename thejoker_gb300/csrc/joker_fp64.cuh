@@ -392,7 +392,7 @@ struct AccFx {
             put((uint32_t)(v.lo >> 32));
             put((uint32_t)v.hi);
         });
-        put((uint32_t)orb.bad);
+        put(orb.bad());
         if (JIT) {
             put((uint32_t)pj);
             put((uint32_t)((uint64_t)pj >> 32));
@@ -410,7 +410,7 @@ struct AccFx {
             const int64_t l = (int64_t)get64();
             v.add(l, (int32_t)get());
         });
-        orb.bad |= (int32_t)get();
+        if (get()) orb.far_r = fx::RI_MAX + 1;
         if (JIT) {
             const int64_t p2 = (int64_t)get64();
             times(p2, (int32_t)get());
@@ -495,6 +495,12 @@ __device__ __forceinline__ void stage_epochs_fx(fx::EpochFx *sm, const double *s
 // alone leave SMs idle or the last wave short.
 constexpr int SLICED_BLOCK = 128;
 
+// Blocks per SM the registers are held to: six (80 registers, a few spills
+// outside the epoch loop) against four gave 334 -> 318 us for 2^20 samples x
+// 16 epochs and 105 -> 91 us for 100003 posterior rows; the large systems of
+// the jitter form would spill their sums.
+constexpr int fx_blocks(int L, bool jit) { return jit && L > 3 ? 3 : 6; }
+
 // Shared memory of such a block: a tile of epochs, then the stored states.
 template <int L, bool JIT> constexpr int sliced_smem(int S) {
     const int tile = TILE * (int)sizeof(fx::EpochFx);
@@ -561,7 +567,7 @@ __device__ __noinline__ double fp64_lnl_global(const StarRec &st, const double *
     if (acc.init(st, P, e, om, M0, s)) {
         const double *rec = ep64 + (size_t)st.epoch_off * REC64;
         for (int i = 0; i < st.n_epochs; ++i, rec += REC64) acc.add(load_epoch_fx(rec));
-        if (!acc.orb.bad) return acc.finish(st, P, e);
+        if (!acc.orb.bad()) return acc.finish(st, P, e);
     }
     return fp64_lnl_doubles<L, JIT>(st, ep64, P, e, om, M0, s);
 }
@@ -580,7 +586,7 @@ __device__ __noinline__ double fp64_lnl_warp_t(const StarRec &st, const double *
         for (int i = threadIdx.x & 31; i < st.n_epochs; i += 32)
             fxa.add(load_epoch_fx(rec0 + (size_t)i * REC64));
         fxa.warp_sum();
-        if (!__any_sync(0xffffffffu, fxa.orb.bad)) return fxa.finish(st, P, e);
+        if (!__any_sync(0xffffffffu, fxa.orb.bad())) return fxa.finish(st, P, e);
     }
     Acc64<L, JIT> acc;
     acc.init(st, P, e, om, M0, s);

@@ -35,10 +35,11 @@ namespace joker {
 // The fixed-point form (AccFx), epochs staged in shared memory; a sample that
 // it does not take runs in doubles (fp64_lnl_doubles).  In doubles the FP64
 // pipe bounded it (70-90 FP64 instructions per epoch, 16 cycles of an SM
-// each); in fixed point instruction issue does.  2^20 samples x 16 epochs:
-// 2267 us in doubles, 352 us; 1.5e6 x 40 with the jitter: 9041, 1520 us.
+// each); in fixed point the integer pipes do.  2^20 samples x 16 epochs:
+// 2267 us in doubles, 318 us; 1.5e6 x 40 with the jitter: 9041, 1377 us.
+// What bounds it now is the pipe of the wide integer multiplies (73 % busy).
 template <int L, bool JIT>
-__global__ void __launch_bounds__(SLICED_BLOCK)
+__global__ void __launch_bounds__(SLICED_BLOCK, fx_blocks(L, JIT))
 lnl_fp64_kernel(LnlArgs a, int S) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int per = SLICED_BLOCK / S;                     // samples per pass
@@ -59,7 +60,7 @@ lnl_fp64_kernel(LnlArgs a, int S) {
             if (!sliced_epochs(acc, active && ok, st, a.ep64, smem, S)) continue;
             double lnl = 0.0;
             if (active) {
-                ok = ok && !acc.orb.bad;
+                ok = ok && !acc.orb.bad();
                 lnl = ok ? acc.finish(st, P, e)
                          : fp64_lnl_doubles<L, JIT>(st, a.ep64, P, e, om, M0, s);
                 a.lnl[w.out_off + j] = lnl;

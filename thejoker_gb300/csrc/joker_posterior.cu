@@ -166,9 +166,9 @@ __device__ __noinline__ void posterior_doubles(const StarRec &st, const double *
 // A warp per sample in doubles spent its time
 // on idle lanes -- 40 epochs on 64 lanes, ten FP64 shuffles a sum, the tail on
 // one lane: 100003 rows x 40 epochs, three linear parameters took
-// 4326 us, now 105.
+// 4326 us, now 91.
 template <int L, bool JIT>
-__global__ void __launch_bounds__(SLICED_BLOCK)
+__global__ void __launch_bounds__(SLICED_BLOCK, fx_blocks(L, JIT))
 posterior_kernel(const StarRec *stars, const double *ep64, int star, const double *P,
                  const double *E, const double *OM, const double *M0, const double *S,
                  int64_t stride, const int64_t *rows, int64_t n, int k_clip, double *a, double *A,
@@ -184,7 +184,7 @@ posterior_kernel(const StarRec *stars, const double *ep64, int star, const doubl
     bool ok = acc.init(st, p, e, om, m0, s);
     if (!sliced_epochs(acc, active && ok, st, ep64, smem, slices) || !active) return;
     double *a_out = a + i * L, *A_out = A + i * L * L, *l_out = lnl ? lnl + i : nullptr;
-    if (!ok || acc.orb.bad) {
+    if (!ok || acc.orb.bad()) {
         posterior_doubles<L>(st, ep64, p, e, om, m0, s, k_clip, a_out, A_out, l_out);
         return;
     }
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(256) unmarginalized_kernel(const StarRec *star
 // 4096 orbits x 1001 times took 785 us.
 constexpr int RV_LANE = 8, RV_TIMES = 32 * RV_LANE;
 
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 6)
 rv_elements_kernel(const double *t, int n_t, const double *el, int64_t n, int per_row, double t0,
                    double *rv) {
     const int lane = threadIdx.x & 31;
@@ -385,7 +385,7 @@ rv_elements_kernel(const double *t, int n_t, const double *el, int64_t n, int pe
                 const double m = (double)orb.column((uint64_t)(q + fx::ONE62));
                 out[j] = K * (m * 0x1p-61);
             }
-            ok = !__any_sync(0xffffffffu, orb.bad);
+            ok = !__any_sync(0xffffffffu, orb.bad());
         }
         if (!ok) {
             OrbitF64 o;
