@@ -9,9 +9,12 @@ bring it to the device:
   rows directly through the chunk's mapped device address and prepares each
   sample in registers (a cache view, ``PriorCache.view``).  The host link
   streams 40 bytes per sample while the kernel computes; there is no staging
-  copy, no preparation pass and no device copy of the chunk.  The FP64
-  re-evaluations of the acceptance pass read the few rows they need the same
-  way.
+  copy, no preparation pass and no device copy of the chunk.  With several
+  stars that would stream the chunk once per star, and the link (211 GB/s) is
+  the bound: slices then go over it once, double-buffered on a copy stream,
+  and the kernel reads the packed rows of a slice for every star from device
+  memory.  The FP64 re-evaluations of the acceptance pass read the few rows
+  they need from the host chunk.
 - staged: the chunk is copied in slices of ``slice_rows`` rows on a copy
   stream, double-buffered, while the previous slice is prepared into a device
   cache and evaluated on a compute stream.
@@ -26,6 +29,20 @@ import torch
 from . import device as dev
 
 __all__ = ["HostRejection"]
+
+# Rows of the slices that several stars share: the first is small, for nothing
+# hides its copy, the later ones are the longest the two buffers hold.
+SHARE_FIRST, SHARE_ROWS = 1 << 18, 1 << 20
+
+
+def _shares(n_stars, rows):
+    """Whether slices pay: the repeated reads that they spare against their
+    launches.  Measured, one read per star -> slices: 4 x 61584 rows 446 ->
+    466 us, 6 x 124776 537 -> 495, 4 x 2^18 591 -> 507, 4 x 2^20 1168 -> 928; two
+    stars, whose second read the kernel mostly covers, 2^20 746 -> 763, 2^22
+    2084 -> 1871."""
+    spared = (n_stars - 1) * rows * 40
+    return spared >= (16 << 20 if n_stars > 2 else 64 << 20)
 
 
 class HostRejection:
@@ -46,9 +63,11 @@ class HostRejection:
         self.chunk = int(chunk)
         n = table.n_stars
         self.cache = None if self.zero_copy else dev.PriorCache(self.capacity)
-        self.stage = [] if self.zero_copy else \
-            [torch.empty((self.slice_rows, 5), dtype=torch.float64, device="cuda")
-             for _ in range(2)]
+        rows = self.slice_rows
+        if self.zero_copy:                     # slices shared by several stars
+            rows = min(SHARE_ROWS, self.capacity) if _shares(n, self.capacity) else 0
+        self.stage = [torch.empty((rows, 5), dtype=torch.float64, device="cuda")
+                      for _ in range(2 if rows else 0)]
         self.lnl = torch.empty((n, self.capacity), dtype=torch.float64, device="cuda")
         mixed = precision != "fp64"
         self.err = torch.empty((n, self.capacity), dtype=torch.float32, device="cuda") \
@@ -80,6 +99,30 @@ class HostRejection:
             dev.lnl(self.table, cache, self.lnl, precision=self.precision, row0=row0,
                     count=count, max_keys=self.keys, err=self.err, bound_keys=self.bkeys,
                     out_offset=row0, chunk=self.chunk, stream=ks)
+
+    def _shared(self, host_chunk, S, ks):
+        """Every star's ln L from slices that cross the link once.  The plain
+        kernel, fused or not: over slices the fused one's longer acceptance
+        costs more than it spares (2 stars x 2^22 rows 2494 us against 1871).
+        Items of at most 512 samples fill the short launches."""
+        cs = self.copy_stream
+        cs.wait_stream(ks)
+        a, k = 0, 0
+        while a < S:
+            b = min(S, a + min(SHARE_FIRST << k, SHARE_ROWS))
+            buf = self.stage[k % 2][: b - a]
+            with torch.cuda.stream(cs):
+                if k >= 2:
+                    cs.wait_event(self.freed[k % 2])
+                buf.copy_(host_chunk[a:b], non_blocking=True)
+                self.copied[k % 2].record(cs)
+            with torch.cuda.stream(ks):
+                ks.wait_event(self.copied[k % 2])
+                dev.lnl(self.table, dev.PriorCache.view(buf), self.lnl, precision=self.precision,
+                        max_keys=self.keys, err=self.err, bound_keys=self.bkeys, out_offset=a,
+                        chunk=min(self.chunk, 512), stream=ks)
+                self.freed[k % 2].record(ks)
+            a, k = b, k + 1
 
     def _staged(self, host_chunk, S, ks, pcg):
         cs = self.copy_stream
@@ -121,13 +164,19 @@ class HostRejection:
                 self.bkeys.t.zero_()
         n = self.table.n_stars
         pcg = None
-        if self.fused:
+        shared = bool(self.zero_copy and self.stage) and _shares(n, S)
+        fused = self.fused and not shared
+        if fused:
             with torch.cuda.stream(ks):
                 pcg = dev.pcg_table([pcg_states[s] for s in range(n)])
         if self.zero_copy:
-            cache = dev.PriorCache.view(host_chunk.contiguous())
-            with torch.cuda.stream(ks):
-                self._lnl(cache, 0, S, pcg, ks)
+            host_chunk = host_chunk.contiguous()
+            cache = dev.PriorCache.view(host_chunk)
+            if shared:
+                self._shared(host_chunk, S, ks)
+            else:
+                with torch.cuda.stream(ks):
+                    self._lnl(cache, 0, S, pcg, ks)
         else:
             cache = self._staged(host_chunk, S, ks, pcg)
         segs = []
@@ -140,7 +189,7 @@ class HostRejection:
             if self.err is None:
                 dev.accept(self.lnl.view(-1), self.keys, segs, out_idx=self.out_idx,
                            counts=self.counts, stream=ks)
-            elif self.fused:
+            elif fused:
                 dev.accept_fused(self.table, cache, self.lnl.view(-1), self.err.view(-1),
                                  self.bkeys, self.cand, self.cand_ld, segs,
                                  out_idx=self.out_idx, counts=self.counts, stream=ks)
