@@ -29,6 +29,7 @@ extern "C" int column(int tsh, int64_t t0, double P, double e, double om, double
 extern "C" int64_t quotient(int64_t num, int64_t den) { return div61(num, den); }
 extern "C" int64_t root(int64_t y) { return sqrt62(y); }
 extern "C" uint64_t inverse(uint64_t dn) { return rcp62(dn); }
+extern "C" double power(int n, int64_t f) { return exp2_fixed(n, f); }
 """
 
 
@@ -46,6 +47,7 @@ def host(tmp_path_factory):
     lib.quotient.argtypes, lib.quotient.restype = [i64, i64], i64
     lib.root.argtypes, lib.root.restype = [i64], i64
     lib.inverse.argtypes, lib.inverse.restype = [u64], u64
+    lib.power.argtypes, lib.power.restype = [ctypes.c_int, i64], dbl
     return lib
 
 
@@ -123,3 +125,17 @@ def test_small_steps(host):
         assert abs(host.root(y) ** 2 - y * one62) <= 2 ** -51.0 * y * one62
         dn = int(rng.integers(one61, one62))
         assert abs(host.inverse(dn) * dn - (1 << 124)) <= 2 ** -57.0 * 2.0 ** 124
+
+
+def test_powers_of_two(host):
+    """2^(n + f): half an ulp of the rounding and the series' 2^-57."""
+    mp = mpmath.mp
+    mp.dps = 40
+    rng = np.random.default_rng(7)
+    one62 = 1 << 62
+    for k in range(2000):
+        f = [0, one62 - 1, (1 << 54) - 1, 1 << 54][k] if k < 4 else int(rng.integers(0, one62))
+        n = int(rng.integers(-1000, 1000)) if k % 2 else 0
+        got, want = mp.mpf(host.power(n, f)), mp.mpf(2) ** (n + mp.mpf(f) / one62)
+        assert abs(got - want) <= mp.mpf(2) ** (n - 53) + want * mp.mpf(2) ** -57
+    assert host.power(3, 0) == 8.0

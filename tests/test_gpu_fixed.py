@@ -100,3 +100,31 @@ def test_rv_curves(cuda, rows, times):
     want = K[:, None] * rv_unit_columns(t, t0, c[:, 0], c[:, 1], c[:, 2], c[:, 3])
     tol = 1e-9 * K / (1.0 - c[:, 1]) ** 2
     assert np.all(np.abs(got.cpu().numpy() - want) <= tol[:, None])
+
+
+@pytest.mark.parametrize("lo,hi", [(2.0, 1024.0), (2.0, 2.0000001), (1e-300, 1e300),
+                                   (1e-310, 1e-300)])
+def test_period_draws(cuda, lo, hi):
+    """P = P_min (P_max / P_min)^u over narrow, ordinary and extreme ranges, the
+    last through doubles; 60 ulps of exp's argument at 700."""
+    from thejoker_gb300 import _native as nat
+    from thejoker_gb300 import device as dev
+    n, seed = 5000, 99
+    packed = torch.empty((n, 5), dtype=torch.float64, device="cuda")
+    dev.PriorCache(n).sample_prior(
+        dict(P_min=lo, P_max=hi, e_alpha=0.867, e_beta=3.03, s_kind=nat.JOKER_S_FIXED,
+             s_value=0.0), n, seed=seed, packed=packed)
+    P = packed[:, 0].cpu().numpy()
+    assert np.all((P >= lo * (1 - 1e-13)) & (P <= hi * (1 + 1e-13)))
+    # the stream's first uniform: Philox4x32-10 of counter (g, 0, 0, tag)
+    g = np.arange(n, dtype=np.uint64)
+    c = [g, 0 * g, 0 * g, 0 * g + np.uint64(0x4A6F6B72)]
+    k, low = [np.uint64(seed), np.uint64(0)], np.uint64(0xFFFFFFFF)
+    for _ in range(10):
+        p0, p1 = c[0] * np.uint64(0xD2511F53), c[2] * np.uint64(0xCD9E8D57)
+        c = [(p1 >> np.uint64(32)) ^ c[1] ^ k[0], p1 & low, (p0 >> np.uint64(32)) ^ c[3] ^ k[1],
+             p0 & low]
+        k = [(k[0] + np.uint64(0x9E3779B9)) & low, (k[1] + np.uint64(0xBB67AE85)) & low]
+    u = (((c[1] << np.uint64(32)) | c[0]) >> np.uint64(11)).astype(np.float64) * 2.0 ** -53
+    want = np.exp(np.log(lo) + u * (np.log(hi) - np.log(lo)))
+    np.testing.assert_allclose(P, want, rtol=60 * 2.0 ** -53 * 700)

@@ -1,9 +1,9 @@
-"""Writes joker_trig_table.cuh: sin and cos of 2 pi k / 2048, k = 0..1024, as
-integers at scale 2^61, each the integer nearest to the exact value (60-digit
-mpmath evaluation).
+"""Writes joker_trig_table.cuh: sin and cos of 2 pi k / 2048, k = 0..1024, and
+2^(k / 512), k = 0..511, as integers at scale 2^61, each the integer nearest to
+the exact value (60-digit mpmath evaluation).
 
-The fixed-point Kepler solver starts its sin and cos series from these nodes.
-Run from any directory:
+The fixed-point Kepler solver starts its sin and cos series from these nodes,
+the period draws their exponential series.  Run from any directory:
 
     python thejoker_gb300/csrc/gen_trig_table.py
 """
@@ -22,8 +22,11 @@ def main():
         s, c = (int(mpmath.nint(v * mpmath.mpf(2) ** 61)) for v in (mpmath.sin(a), mpmath.cos(a)))
         rows.append(f"    {{{s}LL, {c}LL}},")
     body = "\n".join(rows)
+    powers = "\n".join(f"    {int(mpmath.nint(mpmath.mpf(2) ** (61 + mpmath.mpf(k) / 512)))}LL,"
+                       for k in range(512))
     text = f"""// Generated by gen_trig_table.py: sin and cos of 2 pi k / 2048, k = 0..{N - 1},
-// times 2^61, each the nearest integer.  Do not edit.
+// and 2^(k / 512), k = 0..511, times 2^61, each the nearest integer.  Do not
+// edit.
 #pragma once
 #include <cstdint>
 
@@ -40,6 +43,14 @@ static __device__ const trig_entry kTrig[TRIG_N] = {{
 static const trig_entry kTrig[TRIG_N] = {{
 #endif
 {body}
+}};
+
+#ifdef __CUDACC__
+static __device__ const long long kExp2[512] = {{
+#else
+static const long long kExp2[512] = {{
+#endif
+{powers}
 }};
 
 }}  // namespace fx

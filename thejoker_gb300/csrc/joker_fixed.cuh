@@ -32,6 +32,7 @@ constexpr int64_t ONE61 = (int64_t)1 << 61;
 constexpr int64_t ONE62 = (int64_t)1 << 62;
 constexpr int64_t PI_4_Q62 = 0x3243F6A8885A308D;
 constexpr int32_t PI_4_H = (int32_t)(PI_4_Q62 >> 31), PI_4_L = (int32_t)(PI_4_Q62 & 0x7fffffff);
+constexpr int64_t LN2_Q62 = 0x2C5C85FDF473DE6A;
 constexpr uint64_t INV_2PI_Q66 = 0xA2F9836E4E44152Aull, INV_2PI_Q64 = 0x28BE60DB9391054Aull;
 constexpr float TWO_PI_FX = 6.28318530717958648f;
 
@@ -68,6 +69,13 @@ JOKER_FX int32_t hi32(int32_t a, int32_t b) {
     return __mulhi(a, b);
 #else
     return (int32_t)(wide(a, b) >> 32);
+#endif
+}
+JOKER_FX uint32_t uhi32(uint32_t a, uint32_t b) {
+#ifdef __CUDA_ARCH__
+    return __umulhi(a, b);
+#else
+    return (uint32_t)(((uint64_t)a * b) >> 32);
 #endif
 }
 // a b 2^-62 to 5 units (truncated): Qi x Qj -> Q(i + j - 62).  The sum of the
@@ -161,6 +169,15 @@ JOKER_FX uint64_t bits_of(double x) {
     return b;
 #endif
 }
+JOKER_FX double double_of(uint64_t b) {
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double((long long)b);
+#else
+    double x;
+    std::memcpy(&x, &b, 8);
+    return x;
+#endif
+}
 JOKER_FX uint32_t float_bits(float x) {
 #ifdef __CUDA_ARCH__
     return __float_as_uint(x);
@@ -229,6 +246,30 @@ JOKER_FX int64_t sqrt62(int64_t y) {
     const uint32_t s1 = (uint32_t)s + (uint32_t)rint_a(to_float(y - wide(s, s)) * 0.5f * h * 0x1p-31f);
     s = (int32_t)(s1 > 0x7fffffffu ? 0x7fffffffu : s1);   // y near 1: at most 2^31 - 1
     return ((int64_t)s << 31) + (int64_t)rint_a(to_float(y - wide(s, s)) * 0.5f * h);
+}
+
+// 2^(n + f) for f (Q62) in [0, 1) and a normal result: 2^(j/512) times
+// e^z = 1 + z + z^2/2 + z^3 (1/6 + z/24 + z^2/120), z < 2^-9.5, good to 2^-58
+// before the rounding to a double (the truncations leave 0 to -16 units of
+// Q61; 7 are added).
+JOKER_FX double exp2_fixed(int n, int64_t f) {
+#ifdef __CUDA_ARCH__
+    const limbs T = split(__ldg(kExp2 + (int)(f >> 53)));
+#elif defined(__CUDACC__)
+    const limbs T = split(0);            // no host caller
+#else
+    const limbs T = split(kExp2[f >> 53]);
+#endif
+    const limbs z = split(mul(split(f & (((int64_t)1 << 53) - 1)), split(LN2_Q62)));
+    const int64_t zq = join(z);
+    const uint32_t zz = (uint32_t)(zq >> 21);                        // 2^41 z
+    const float zf = (float)zz * 0x1p-41f;
+    const uint32_t h = 2863311531u +                                 // 2^34 / 6
+                       (uint32_t)rint_a(zf * fma_a(zf, 1.0f / 120.0f, 1.0f / 24.0f) * 0x1p34f);
+    const uint32_t z3 = uhi32(uhi32(zz, zz), zz);                    // 2^59 z^3
+    const int64_t p = zq + (mul(z, z) >> 1) + 2 * (int64_t)uhi32(z3, h);
+    const int64_t v = join(T) + mul(T, split(p));                    // Q61, [1, 2)
+    return double_of(((uint64_t)(1022 + n) << 52) + (uint64_t)((v + 263) >> 9));
 }
 
 // One orbit against one star's time scale.
