@@ -62,6 +62,7 @@ struct joker_stars {
     float *d_ep32 = nullptr;
     int *d_queue = nullptr;
     int *d_order = nullptr;      // stars sorted by epoch count, largest first
+    void *base = nullptr;        // the one allocation that holds them all
 };
 
 struct joker_cache {
@@ -72,6 +73,44 @@ struct joker_cache {
     float4 *mx_a = nullptr, *mx_b = nullptr;
     float *mx_s2 = nullptr;
     int *flag = nullptr;         // device word for joker_prior_sample's status
+    void *base = nullptr;        // the one allocation that holds the columns it owns
+};
+
+// Offsets of the parts of one allocation, each on a 256-byte boundary.  One
+// cudaMalloc and one cudaFree (which waits for the device) per handle: a table
+// of five parts and a cache of nine cost a small call 0.7 ms.
+struct Parts {
+    size_t total = 0;
+    size_t take(size_t bytes) {
+        const size_t at = total;
+        total += (bytes + 255) & ~(size_t)255;
+        return at;
+    }
+};
+
+// Where a star table's parts lie; the first four are what the host fills.
+struct StarParts {
+    Parts p;
+    size_t stars, ep64, ep32, order, filled, queue;
+    StarParts(int n_stars, int64_t epochs) {
+        stars = p.take(sizeof(StarRec) * (size_t)n_stars);
+        ep64 = p.take(sizeof(double) * REC64 * (size_t)epochs);
+        ep32 = p.take(sizeof(float) * REC32 * (size_t)epochs);
+        order = p.take(sizeof(int) * (size_t)n_stars);
+        filled = p.total;
+        queue = p.take(sizeof(int) * 4);
+    }
+    cudaError_t allocate(joker_stars *s) const {
+        const cudaError_t e = cudaMalloc(&s->base, p.total);
+        if (e != cudaSuccess) return e;
+        char *b = (char *)s->base;
+        s->d_stars = (StarRec *)(b + stars);
+        s->d_ep64 = (double *)(b + ep64);
+        s->d_ep32 = (float *)(b + ep32);
+        s->d_order = (int *)(b + order);
+        s->d_queue = (int *)(b + queue);
+        return cudaSuccess;
+    }
 };
 
 namespace joker {
@@ -470,9 +509,12 @@ extern "C" int joker_stars_create(joker_stars **out, int n_stars, int n_linear,
         max_ep = std::max<int>(max_ep, (int)n);
     }
     const int64_t NE = epoch_offsets[n_stars];
-    std::vector<StarRec> recs(n_stars);
-    std::vector<double> ep64((size_t)NE * REC64, 0.0);
-    std::vector<float> ep32((size_t)NE * REC32, 0.0f);
+    const StarParts parts(n_stars, NE);
+    std::vector<char> host(parts.filled, 0);                 // the table as it goes to the device
+    StarRec *recs = (StarRec *)(host.data() + parts.stars);
+    double *ep64 = (double *)(host.data() + parts.ep64);
+    float *ep32 = (float *)(host.data() + parts.ep32);
+    int *order = (int *)(host.data() + parts.order);
     for (int k = 0; k < n_stars; ++k) {
         const int64_t e0 = epoch_offsets[k];
         const int n = (int)(epoch_offsets[k + 1] - e0);
@@ -483,9 +525,8 @@ extern "C" int joker_stars_create(joker_stars **out, int n_stars, int n_linear,
                                  recs[k], &ep64[(size_t)e0 * REC64], &ep32[(size_t)e0 * REC32]);
         if (rc != JOKER_OK) return rc;
     }
-    std::vector<int> order(n_stars);
     for (int k = 0; k < n_stars; ++k) order[k] = k;
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    std::stable_sort(order, order + n_stars, [&](int a, int b) {
         return recs[a].n_epochs > recs[b].n_epochs;
     });
 
@@ -496,26 +537,16 @@ extern "C" int joker_stars_create(joker_stars **out, int n_stars, int n_linear,
     s->max_epochs = max_ep;
     s->total_epochs = NE;
     s->off.assign(epoch_offsets, epoch_offsets + n_stars + 1);
-    for (const StarRec &r : recs) s->fixed.push_back(r.fx_ok && r.mu0 == 0.0);
-    auto cleanup = [&]() { joker_stars_destroy(s); };
-    cudaError_t e;
-    if ((e = cudaMalloc(&s->d_stars, sizeof(StarRec) * n_stars)) != cudaSuccess ||
-        (e = cudaMalloc(&s->d_ep64, sizeof(double) * ep64.size())) != cudaSuccess ||
-        (e = cudaMalloc(&s->d_ep32, sizeof(float) * ep32.size())) != cudaSuccess ||
-        (e = cudaMalloc(&s->d_queue, sizeof(int) * 4)) != cudaSuccess ||
-        (e = cudaMalloc(&s->d_order, sizeof(int) * n_stars)) != cudaSuccess) {
-        cleanup();
+    for (int k = 0; k < n_stars; ++k)
+        s->fixed.push_back(recs[k].fx_ok && recs[k].mu0 == 0.0);
+    cudaError_t e = parts.allocate(s);
+    if (e != cudaSuccess) {
+        joker_stars_destroy(s);
         return fail(JOKER_ENOMEM, "joker_stars_create: cudaMalloc: %s", cudaGetErrorString(e));
     }
-    if ((e = cudaMemcpy(s->d_stars, recs.data(), sizeof(StarRec) * n_stars,
-                        cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMemcpy(s->d_ep64, ep64.data(), sizeof(double) * ep64.size(),
-                        cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMemcpy(s->d_ep32, ep32.data(), sizeof(float) * ep32.size(),
-                        cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMemcpy(s->d_order, order.data(), sizeof(int) * n_stars,
-                        cudaMemcpyHostToDevice)) != cudaSuccess) {
-        cleanup();
+    if ((e = cudaMemcpy(s->base, host.data(), parts.filled, cudaMemcpyHostToDevice)) !=
+        cudaSuccess) {
+        joker_stars_destroy(s);
         return fail(JOKER_ECUDA, "joker_stars_create: cudaMemcpy: %s", cudaGetErrorString(e));
     }
     *out = s;
@@ -553,11 +584,7 @@ extern "C" int joker_stars_create_slots(joker_stars **out, int n_slots, int max_
     std::vector<int> order(n_slots);
     for (int k = 0; k < n_slots; ++k) order[k] = k;
     cudaError_t e;
-    if ((e = cudaMalloc(&s->d_stars, sizeof(StarRec) * n_slots)) != cudaSuccess ||
-        (e = cudaMalloc(&s->d_ep64, sizeof(double) * REC64 * s->total_epochs)) != cudaSuccess ||
-        (e = cudaMalloc(&s->d_ep32, sizeof(float) * REC32 * s->total_epochs)) != cudaSuccess ||
-        (e = cudaMalloc(&s->d_queue, sizeof(int) * 4)) != cudaSuccess ||
-        (e = cudaMalloc(&s->d_order, sizeof(int) * n_slots)) != cudaSuccess ||
+    if ((e = StarParts(n_slots, s->total_epochs).allocate(s)) != cudaSuccess ||
         (e = cudaMemcpy(s->d_stars, recs.data(), sizeof(StarRec) * n_slots,
                         cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemcpy(s->d_order, order.data(), sizeof(int) * n_slots,
@@ -606,11 +633,7 @@ extern "C" int joker_stars_set(joker_stars *s, int slot, int n_epochs, const dou
 
 extern "C" int joker_stars_destroy(joker_stars *s) {
     if (!s) return JOKER_OK;
-    cudaFree(s->d_stars);
-    cudaFree(s->d_ep64);
-    cudaFree(s->d_ep32);
-    cudaFree(s->d_queue);
-    cudaFree(s->d_order);
+    cudaFree(s->base);
     delete s;
     return JOKER_OK;
 }
@@ -632,29 +655,37 @@ extern "C" int joker_cache_create(joker_cache **out, int64_t capacity) {
     if (capacity <= 0) return fail(JOKER_EINVAL, "joker_cache_create: capacity must be > 0");
     joker_cache *c = new joker_cache();
     c->cap = capacity;
-    cudaError_t e;
     const size_t n = (size_t)capacity;
-    if ((e = cudaMalloc(&c->P, 8 * n)) != cudaSuccess || (e = cudaMalloc(&c->E, 8 * n)) != cudaSuccess ||
-        (e = cudaMalloc(&c->OM, 8 * n)) != cudaSuccess || (e = cudaMalloc(&c->M0, 8 * n)) != cudaSuccess ||
-        (e = cudaMalloc(&c->S, 8 * n)) != cudaSuccess ||
-        (e = cudaMalloc(&c->mx_a, 16 * n)) != cudaSuccess ||
-        (e = cudaMalloc(&c->mx_b, 16 * n)) != cudaSuccess ||
-        (e = cudaMalloc(&c->mx_s2, 4 * n)) != cudaSuccess ||
-        (e = cudaMalloc(&c->flag, sizeof(int))) != cudaSuccess) {
+    Parts p;
+    const size_t col[5] = {p.take(8 * n), p.take(8 * n), p.take(8 * n), p.take(8 * n),
+                           p.take(8 * n)};
+    const size_t a = p.take(16 * n), b = p.take(16 * n), s2 = p.take(4 * n),
+                 flag = p.take(sizeof(int));
+    // (a capacity whose bytes would not fit in size_t is more than any memory)
+    const cudaError_t e = capacity >> 48 ? cudaErrorMemoryAllocation
+                                         : cudaMalloc(&c->base, p.total);
+    if (e != cudaSuccess) {
         joker_cache_destroy(c);
         return fail(JOKER_ENOMEM, "joker_cache_create(%lld): %s", (long long)capacity,
                     cudaGetErrorString(e));
     }
+    char *base = (char *)c->base;
+    c->P = (double *)(base + col[0]);
+    c->E = (double *)(base + col[1]);
+    c->OM = (double *)(base + col[2]);
+    c->M0 = (double *)(base + col[3]);
+    c->S = (double *)(base + col[4]);
+    c->mx_a = (float4 *)(base + a);
+    c->mx_b = (float4 *)(base + b);
+    c->mx_s2 = (float *)(base + s2);
+    c->flag = (int *)(base + flag);
     *out = c;
     return JOKER_OK;
 }
 
 extern "C" int joker_cache_destroy(joker_cache *c) {
     if (!c) return JOKER_OK;
-    if (!c->view) {
-        cudaFree(c->P); cudaFree(c->E); cudaFree(c->OM); cudaFree(c->M0); cudaFree(c->S);
-    }
-    cudaFree(c->mx_a); cudaFree(c->mx_b); cudaFree(c->mx_s2); cudaFree(c->flag);
+    cudaFree(c->base);                                       // NULL for a view
     delete c;
     return JOKER_OK;
 }
