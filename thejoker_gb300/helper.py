@@ -7,14 +7,22 @@ It exposes the surface the reference's sampling code uses
 by its constructor arguments (``__reduce__``, :122-123).  The likelihood runs
 in libjoker_gb300 on the GPU; there is no CPU path.
 """
+import ctypes
+
 import numpy as np
 import torch
 
+from . import _native as nat
 from . import device as dev
 from .linear import multivariate_normal_draws
 from .samples import PACKED_ORDER
 
 __all__ = ["GPUJokerHelper", "band_refined_lnl"]
+
+# Host calls of up to this many rows let the FP64 kernel read the pinned rows
+# and write the pinned results itself, two copies fewer: 97 rows x 3 epochs 92 ->
+# 60 us, 16384 x 16 155 -> 104; at 65536 the copy engine reads faster (179, 186).
+MAPPED_ROWS = 16384
 
 
 def band_refined_lnl(stars, cache, out, precision, star=0, stream=None):
@@ -93,12 +101,7 @@ class GPUJokerHelper:
         if out is None:
             out = torch.empty(S, dtype=torch.float64, device=chunk.device)
         if self.precision == "fp64":
-            import ctypes
-            from . import _native as nat
-            nat.check(nat.lib().joker_batch_marginal_ln_likelihood(
-                self._stars.handle, 0, ctypes.c_void_p(chunk.data_ptr()), S,
-                ctypes.c_void_p(out.data_ptr()), dev.stream_handle(stream)),
-                "joker_batch_marginal_ln_likelihood")
+            self._fp64_into(chunk, out, stream)
         else:
             cache = dev.PriorCache.from_samples(chunk, stream=stream)
             if self.precision == "mixed_fp64_tail":
@@ -115,11 +118,26 @@ class GPUJokerHelper:
         chunk = np.ascontiguousarray(chunk, dtype=np.float64)
         if chunk.ndim != 2 or chunk.shape[1] != 5:
             raise ValueError("chunk must have shape (n_samples, 5)")
-        if chunk.shape[0] == 0:
+        S = chunk.shape[0]
+        if S == 0:
             return np.zeros(0)
-        d = torch.from_numpy(chunk).pin_memory().to("cuda", non_blocking=True)
-        out = self.batch_marginal_ln_likelihood_device(d)
+        rows = torch.from_numpy(chunk).pin_memory()
+        if self.precision == "fp64" and S <= MAPPED_ROWS:
+            out = torch.empty(S, dtype=torch.float64, pin_memory=True)
+            stream = torch.cuda.current_stream()
+            self._fp64_into(rows, out, stream)
+            stream.synchronize()
+            return out.numpy().copy()      # the pinned block goes back to its pool
+        out = self.batch_marginal_ln_likelihood_device(rows.to("cuda", non_blocking=True))
         return out.cpu().numpy()
+
+    def _fp64_into(self, rows, out, stream=None):
+        """joker_batch_marginal_ln_likelihood: rows and out in device memory, or
+        in pinned memory that the kernel reads and writes over the link."""
+        nat.check(nat.lib().joker_batch_marginal_ln_likelihood(
+            self._stars.handle, 0, ctypes.c_void_p(rows.data_ptr()), rows.shape[0],
+            ctypes.c_void_p(out.data_ptr()), dev.stream_handle(stream)),
+            "joker_batch_marginal_ln_likelihood")
 
     def test_likelihood_worker(self, chunk_row):
         """ln L of one packed sample (fast_likelihood.pyx:547-576)."""
