@@ -358,6 +358,12 @@ int joker_iter_create_pool(joker_iter **out, const joker_stars *stars, const jok
 int joker_iter_admit(joker_iter *it, int slot, int64_t budget, int n_requested,
                      int64_t init_batch, int64_t pool_off, const uint64_t *pcg_state,
                      void *stream);
+
+/* Restart every slot of the handle (between rounds): slot s with its pool
+ * range at s * budget and the stream pcg_states[4 s ..], as joker_iter_admit
+ * for each, in one launch per 100 slots. */
+int joker_iter_restart(joker_iter *it, int64_t budget, int n_requested, int64_t init_batch,
+                       const uint64_t *pcg_states, void *stream);
 /* Samples evaluated per round over all stars (0, the default: no limit).  A
  * star whose batch is larger than its equal share of the budget spreads the
  * batch over several rounds; its acceptance runs once the batch is complete,

@@ -227,10 +227,10 @@ __global__ void iter_update_kernel(IterParams p) {
 
 // Start a request in slot s (between rounds): its schedule, pool buffer and
 // uniform stream; the slot's running maxima are reset.
-__global__ void iter_admit_kernel(IterParams p, unsigned long long *max_key,
-                                  unsigned long long *bound_key, int s, int64_t budget, int n_req,
-                                  int64_t init, int64_t pool_off, uint64_t s_hi, uint64_t s_lo,
-                                  uint64_t i_hi, uint64_t i_lo) {
+__device__ __forceinline__ void admit_slot(IterParams p, unsigned long long *max_key,
+                                           unsigned long long *bound_key, int s, int64_t budget,
+                                           int n_req, int64_t init, int64_t pool_off,
+                                           const uint64_t *pcg) {
     int64_t *st = p.state + (int64_t)s * ST_FIELDS;
     // the finished count covers slots holding a finished request
     if (st[ST_DONE] >= 1 && st[ST_DONE] <= 3) atomicSub(p.done_count, 1);
@@ -240,10 +240,27 @@ __global__ void iter_admit_kernel(IterParams p, unsigned long long *max_key,
     p.n_req[s] = n_req;
     p.lnl_off[s] = pool_off;
     uint64_t *pc = const_cast<uint64_t *>(p.pcg0) + 4 * s;
-    pc[0] = s_hi; pc[1] = s_lo; pc[2] = i_hi; pc[3] = i_lo;
+    for (int k = 0; k < 4; ++k) pc[k] = pcg[k];
     max_key[s] = 0ull;
     bound_key[2 * s] = 0ull;
     bound_key[2 * s + 1] = 0ull;
+}
+
+// Up to ADMIT_BATCH slots from s0 on, one thread each; their streams travel
+// with the launch (3.2 KB of parameters).
+constexpr int ADMIT_BATCH = 100;
+struct AdmitStreams {
+    uint64_t pcg[ADMIT_BATCH][4];
+};
+
+__global__ void __launch_bounds__(128)
+iter_admit_kernel(IterParams p, unsigned long long *max_key, unsigned long long *bound_key, int s0,
+                  int n, int64_t budget, int n_req, int64_t init, int64_t pool_off,
+                  int64_t pool_stride, const __grid_constant__ AdmitStreams streams) {
+    const int k = threadIdx.x;
+    if (k < n)
+        admit_slot(p, max_key, bound_key, s0 + k, budget, n_req, init, pool_off + k * pool_stride,
+                   streams.pcg[k]);
 }
 
 }  // namespace
@@ -410,31 +427,54 @@ static int iter_alloc(joker_iter **out, const joker_stars *stars, const joker_ca
     return JOKER_OK;
 }
 
-extern "C" int joker_iter_admit(joker_iter *it, int slot, int64_t budget, int n_requested,
-                                int64_t init_batch, int64_t pool_off, const uint64_t *pcg_state,
-                                void *stream) {
-    if (!it || !pcg_state) return iter_fail(JOKER_EINVAL, "joker_iter_admit: NULL argument");
-    if (slot < 0 || slot >= it->p.n_stars)
-        return iter_fail(JOKER_EINVAL, "joker_iter_admit: slot out of range");
+// Slots [s0, s0 + n), whose pool ranges follow one another from pool_off on.
+static int admit_slots(joker_iter *it, int s0, int n, int64_t budget, int n_requested,
+                       int64_t init_batch, int64_t pool_off, const uint64_t *pcg_states,
+                       cudaStream_t stream, const char *who) {
+    auto refuse = [who](int code, const char *why) {
+        char buf[256];
+        snprintf(buf, sizeof buf, "%s: %s", who, why);
+        return iter_fail(code, buf);
+    };
+    if (!it || !pcg_states) return refuse(JOKER_EINVAL, "NULL argument");
+    if (s0 < 0 || n < 0 || s0 > it->p.n_stars - n) return refuse(JOKER_EINVAL, "slot out of range");
     int64_t cap, cstride; const double *P, *E, *OM, *M0, *S; const float4 *ma, *mb; const float *ms;
     cache_internals(it->cache, &cap, &P, &E, &OM, &M0, &S, &cstride, &ma, &mb, &ms);
-    if (budget <= 0 || it->p.lib_row0 + budget > cap)
-        return iter_fail(JOKER_ERANGE, "joker_iter_admit: budget outside the cache");
+    if (budget <= 0 || budget > cap - it->p.lib_row0)
+        return refuse(JOKER_ERANGE, "budget outside the cache");
     if (n_requested <= 0 || n_requested > it->p.max_req)
-        return iter_fail(JOKER_ERANGE, "joker_iter_admit: n_requested outside [1, max_req]");
+        return refuse(JOKER_ERANGE, "n_requested outside [1, max_req]");
     if (init_batch <= 0 || init_batch > budget)
         return iter_fail(JOKER_EINVAL, "Prior sample library not big enough! For iterative "
                                        "sampling, you have to have at least growth_factor * "
                                        "n_requested_samples samples in the library.");
-    if (pool_off < 0 || pool_off + budget > it->pool)
-        return iter_fail(JOKER_ERANGE, "joker_iter_admit: pool range outside the pool");
-    iter_admit_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(
-        it->p, it->max_key, it->bound_key, slot, budget, n_requested, init_batch, pool_off,
-        pcg_state[0], pcg_state[1], pcg_state[2], pcg_state[3]);
-    count_launch();
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return iter_fail(JOKER_ECUDA, cudaGetErrorString(e));
+    if (pool_off < 0 || n > it->pool / budget || pool_off > it->pool - n * budget)
+        return refuse(JOKER_ERANGE, "pool range outside the pool");
+    for (int k = 0; k < n; k += ADMIT_BATCH) {
+        AdmitStreams streams;
+        const int m = std::min(n - k, ADMIT_BATCH);
+        memcpy(streams.pcg, pcg_states + 4 * (size_t)k, sizeof(streams.pcg[0]) * m);
+        iter_admit_kernel<<<1, 128, 0, stream>>>(it->p, it->max_key, it->bound_key, s0 + k, m,
+                                                 budget, n_requested, init_batch,
+                                                 pool_off + k * budget, budget, streams);
+        count_launch();
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return iter_fail(JOKER_ECUDA, cudaGetErrorString(e));
+    }
     return JOKER_OK;
+}
+
+extern "C" int joker_iter_admit(joker_iter *it, int slot, int64_t budget, int n_requested,
+                                int64_t init_batch, int64_t pool_off, const uint64_t *pcg_state,
+                                void *stream) {
+    return admit_slots(it, slot, 1, budget, n_requested, init_batch, pool_off, pcg_state,
+                       (cudaStream_t)stream, "joker_iter_admit");
+}
+
+extern "C" int joker_iter_restart(joker_iter *it, int64_t budget, int n_requested,
+                                  int64_t init_batch, const uint64_t *pcg_states, void *stream) {
+    return admit_slots(it, 0, it ? it->p.n_stars : 0, budget, n_requested, init_batch, 0,
+                       pcg_states, (cudaStream_t)stream, "joker_iter_restart");
 }
 
 extern "C" int joker_iter_create_pool(joker_iter **out, const joker_stars *stars,
@@ -470,13 +510,10 @@ extern "C" int joker_iter_create(joker_iter **out, const joker_stars *stars,
     int rc = iter_alloc(&it, stars, cache, precision, lib_row0, lib_size * n_stars, n_requested,
                         safety_factor, maxiter, chunk, "joker_iter_create");
     if (rc != JOKER_OK) return rc;
-    for (int s = 0; s < n_stars; ++s) {
-        rc = joker_iter_admit(it, s, lib_size, n_requested, init_batch, (int64_t)s * lib_size,
-                              pcg_states + 4 * (size_t)s, nullptr);
-        if (rc != JOKER_OK) {
-            joker_iter_destroy(it);
-            return rc;
-        }
+    rc = joker_iter_restart(it, lib_size, n_requested, init_batch, pcg_states, nullptr);
+    if (rc != JOKER_OK) {
+        joker_iter_destroy(it);
+        return rc;
     }
     if (cudaDeviceSynchronize() != cudaSuccess) {
         joker_iter_destroy(it);

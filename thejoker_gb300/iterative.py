@@ -67,19 +67,19 @@ class IterativeBatch:
             raise ValueError("one seed per star")
         pcg = np.zeros((self.n, 4), dtype=np.uint64)
         for k, sd in enumerate(seeds):
-            st, inc = dev.pcg64_state(np.random.default_rng(int(sd)))
+            s = np.random.PCG64(int(sd)).state["state"]      # default_rng's generator
+            st, inc = s["state"], s["inc"]
             pcg[k] = [st >> 64, st & ((1 << 64) - 1), inc >> 64, inc & ((1 << 64) - 1)]
         return pcg
 
     def reset(self, seeds):
-        """Start every star again with new seeds (joker_iter_admit per star);
-        the buffers and a captured round graph stay valid."""
+        """Start every star again with new seeds (joker_iter_restart); the
+        buffers and a captured round graph stay valid."""
         pcg = self._pcg(seeds)
-        st = dev.stream_handle()
-        for k in range(self.n):
-            nat.check(nat.lib().joker_iter_admit(
-                self._h, k, self.lib_size, self.n_requested, self.init, k * self.lib_size,
-                pcg[k].ctypes.data_as(ctypes.POINTER(ctypes.c_uint64)), st), "joker_iter_admit")
+        nat.check(nat.lib().joker_iter_restart(
+            self._h, self.lib_size, self.n_requested, self.init,
+            pcg.ctypes.data_as(ctypes.POINTER(ctypes.c_uint64)), dev.stream_handle()),
+            "joker_iter_restart")
         return self
 
     def _round(self):
