@@ -480,66 +480,47 @@ __global__ void __launch_bounds__(ACC_THREADS) accept_mark_kernel(AcceptArgs a) 
 // sample without it is rejected.  These scans read the bits (1/96 of the
 // bytes of ln L and its bound) and touch ln L only where a bit is set.
 
-__device__ __forceinline__ uint32_t cand_word(const AcceptArgs &a, int si, int64_t n,
-                                              int64_t first) {
-    if (first >= n) return 0u;
-    uint32_t w = a.cand_words[(int64_t)si * a.cand_ld + (first >> 5)];
-    if (n - first < 32) w &= (1u << (n - first)) - 1u;
-    return w;
-}
+// Both scans take 1024 samples -- a part of an 8192-sample CTA block -- per
+// warp (grid-stride): each lane loads one of the part's 32 words of candidate
+// bits, and only the nonzero words are visited, each by the whole warp (lane b
+// on the word's sample b).  The arrays they fill (amb_words, words) and the
+// per-CTA counts are zeroed before; a part without candidate bits costs its
+// load.  A warp per CTA block visited up to 256 words one after another, each a
+// chain of dependent loads: 48 stars x 4e5 samples, where stars of few epochs
+// leave most bits set, took 158 and 176 us for the two scans.
+constexpr int PARTS = ACC_THREADS / 32;
 
-// Both scans take one 8192-sample CTA block per warp (grid-stride): each lane
-// loads 8 of the block's 256 words of candidate bits (two 16-byte loads, all
-// independent), and only the nonzero words are visited, each by the whole
-// warp (lane b on the word's sample b).  The arrays they fill (amb_words,
-// words) and the per-CTA counts are zeroed before; a block without candidate
-// bits costs its loads.
-struct FusedBlock {
+struct FusedPart {
     int si;
     joker_accept_seg sg;
-    int64_t gblk, first;      // CTA block; its first sample in the segment
-    uint32_t wv[8];           // words 8 lane .. 8 lane + 7 of the block
+    int64_t gblk, block_first;   // CTA block; its first sample in the segment
+    int w0;                      // the part's first word in the block
+    uint32_t bits;               // word w0 + lane
 };
 
-__device__ __forceinline__ void fused_block(const AcceptArgs &a, int64_t gblk, FusedBlock &b) {
-    const int lane = threadIdx.x & 31;
-    b.gblk = gblk;
-    b.si = find_seg(a, gblk);
+__device__ __forceinline__ void fused_part(const AcceptArgs &a, int64_t unit, FusedPart &b) {
+    b.gblk = unit / PARTS;
+    b.w0 = (int)(unit % PARTS) * 32;
+    b.si = find_seg(a, b.gblk);
     b.sg = a.segs[b.si];
-    b.first = (gblk - seg_base(a, b.si)) * ACC_BLOCK;
-    const int64_t nw = (b.sg.n + 31) >> 5;                  // words of the segment
-    const int64_t w0 = (b.first >> 5) + 8 * lane;
-    const uint32_t *row = a.cand_words + (int64_t)b.si * a.cand_ld;
-    if (w0 + 8 <= nw) {
-        const uint4 p = *reinterpret_cast<const uint4 *>(row + w0);
-        const uint4 q = *reinterpret_cast<const uint4 *>(row + w0 + 4);
-        b.wv[0] = p.x; b.wv[1] = p.y; b.wv[2] = p.z; b.wv[3] = p.w;
-        b.wv[4] = q.x; b.wv[5] = q.y; b.wv[6] = q.z; b.wv[7] = q.w;
-    } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) b.wv[j] = w0 + j < nw ? row[w0 + j] : 0u;
-    }
-    // the segment's last word: bits past its last sample
-    const int64_t tail = b.sg.n & 31;
-    if (tail) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            if (w0 + j == nw - 1) b.wv[j] &= (1u << tail) - 1u;
-    }
+    b.block_first = (b.gblk - seg_base(a, b.si)) * ACC_BLOCK;
+    // the row's word first, whatever the segment's length (one wait fewer)
+    const int64_t first = b.block_first + 32 * (b.w0 + (threadIdx.x & 31));
+    const uint32_t w =
+        (first >> 5) < a.cand_ld ? a.cand_words[(int64_t)b.si * a.cand_ld + (first >> 5)] : 0u;
+    const int64_t left = b.sg.n - first;
+    b.bits = left >= 32 ? w : left > 0 ? w & ((1u << left) - 1u) : 0u;
 }
 
-// Visit every nonzero word of the block: fn(word index in the block, bits),
+// Visit every nonzero word of the part: fn(word index in the block, bits),
 // called by all lanes (warp-uniform).
 template <class F>
-__device__ __forceinline__ void for_nonzero_words(const FusedBlock &b, F fn) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        unsigned owners = __ballot_sync(0xffffffffu, b.wv[j] != 0u);
-        while (owners) {
-            const int l = __ffs(owners) - 1;
-            owners &= owners - 1;
-            fn(8 * l + j, __shfl_sync(0xffffffffu, b.wv[j], l));
-        }
+__device__ __forceinline__ void for_nonzero_words(const FusedPart &b, F fn) {
+    unsigned owners = __ballot_sync(0xffffffffu, b.bits != 0u);
+    while (owners) {
+        const int l = __ffs(owners) - 1;
+        owners &= owners - 1;
+        fn(b.w0 + l, __shfl_sync(0xffffffffu, b.bits, l));
     }
 }
 
@@ -550,13 +531,13 @@ __device__ __forceinline__ void for_nonzero_words(const FusedBlock &b, F fn) {
 __global__ void __launch_bounds__(ACC_THREADS) fused_max_cands_kernel(AcceptArgs a, int64_t nbk) {
     const int lane = threadIdx.x & 31;
     const int64_t nwarps = (int64_t)gridDim.x * (ACC_THREADS / 32);
-    for (int64_t gblk = blockIdx.x * (int64_t)(ACC_THREADS / 32) + (threadIdx.x >> 5);
-         gblk < nbk; gblk += nwarps) {
-        FusedBlock b;
-        fused_block(a, gblk, b);
+    for (int64_t unit = blockIdx.x * (int64_t)(ACC_THREADS / 32) + (threadIdx.x >> 5);
+         unit < nbk * PARTS; unit += nwarps) {
+        FusedPart b;
+        fused_part(a, unit, b);
         const double lb = key_to_double(a.bound_key[2 * b.sg.max_slot + 1]);
         for_nonzero_words(b, [&](int w, uint32_t bits) {
-            const int64_t i = b.first + 32 * w + lane;
+            const int64_t i = b.block_first + 32 * w + lane;
             bool cand = false;
             if ((bits >> lane) & 1u) {
                 const double v = a.lnl[b.sg.lnl_off + i];
@@ -564,7 +545,7 @@ __global__ void __launch_bounds__(ACC_THREADS) fused_max_cands_kernel(AcceptArgs
                 cand = (v + (double)er >= lb) || !(er < 1e29f) || !(v == v);
             }
             const uint32_t over = __ballot_sync(0xffffffffu, !flag_append(a, 0, cand, b.si, i));
-            if (over && lane == 0) a.amb_words[gblk * ACC_THREADS + w] = over;
+            if (over && lane == 0) a.amb_words[b.gblk * ACC_THREADS + w] = over;
         });
     }
 }
@@ -578,26 +559,23 @@ __global__ void __launch_bounds__(ACC_THREADS) fused_max_cands_kernel(AcceptArgs
 __global__ void __launch_bounds__(ACC_THREADS) fused_decide_kernel(AcceptArgs a, int64_t nbk) {
     const int lane = threadIdx.x & 31;
     const int64_t nwarps = (int64_t)gridDim.x * (ACC_THREADS / 32);
-    for (int64_t gblk = blockIdx.x * (int64_t)(ACC_THREADS / 32) + (threadIdx.x >> 5);
-         gblk < nbk; gblk += nwarps) {
-        FusedBlock b;
-        fused_block(a, gblk, b);
-        bool any = false;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) any |= b.wv[j] != 0u;
-        if (!__any_sync(0xffffffffu, any)) continue;
+    for (int64_t unit = blockIdx.x * (int64_t)(ACC_THREADS / 32) + (threadIdx.x >> 5);
+         unit < nbk * PARTS; unit += nwarps) {
+        FusedPart b;
+        fused_part(a, unit, b);
+        if (!__any_sync(0xffffffffu, b.bits != 0u)) continue;
         const double mx = key_to_double(a.exact_key[b.sg.max_slot]);
         float mxf;
         const bool fast = dbl_to_float_trunc(mx, mxf);
         const u128 inc = ((u128)b.sg.pcg_inc_hi << 64) | (u128)b.sg.pcg_inc_lo;
         const u128 sblk = pcg_jump(((u128)b.sg.pcg_state_hi << 64) | (u128)b.sg.pcg_state_lo, inc,
-                                   (uint64_t)b.first);
+                                   (uint64_t)b.block_first);
         const unsigned long long *lt = g_pcg_thr.v[lane];
         const u128 a_lane = ((u128)lt[1] << 64) | (u128)lt[0];
         const u128 c_lane = (((u128)lt[3] << 64) | (u128)lt[2]) * inc;
         int count = 0;
         for_nonzero_words(b, [&](int w, uint32_t bits) {
-            const int64_t i = b.first + 32 * w + lane;
+            const int64_t i = b.block_first + 32 * w + lane;
             const unsigned long long *wt = g_pcg_w32.v[w];
             const u128 sw = (((u128)wt[1] << 64) | (u128)wt[0]) * sblk +
                             (((u128)wt[3] << 64) | (u128)wt[2]) * inc;
@@ -617,13 +595,13 @@ __global__ void __launch_bounds__(ACC_THREADS) fused_decide_kernel(AcceptArgs a,
             const uint32_t bal = __ballot_sync(0xffffffffu, keep);
             const uint32_t over = __ballot_sync(0xffffffffu, !flag_append(a, 1, amb, b.si, i));
             if (lane == 0) {
-                if (bal) a.words[gblk * ACC_THREADS + w] = bal;
-                if (over) a.amb_words[gblk * ACC_THREADS + w] = over;
+                if (bal) a.words[b.gblk * ACC_THREADS + w] = bal;
+                if (over) a.amb_words[b.gblk * ACC_THREADS + w] = over;
             }
             count += __popc(bal);
         });
         if (lane == 0 && count)
-            atomicAdd((unsigned long long *)(a.blk_count + gblk), (unsigned long long)count);
+            atomicAdd((unsigned long long *)(a.blk_count + b.gblk), (unsigned long long)count);
     }
 }
 
@@ -682,19 +660,38 @@ __global__ void __launch_bounds__(SCAN_THREADS) accept_scan_kernel(AcceptArgs a)
 // on flag list 0 for re-evaluation in FP64 (or, past the list's capacity,
 // re-evaluated here), so that every ln L written out is within that of FP64.
 template <bool FLAG>
-__global__ void __launch_bounds__(ACC_THREADS) accept_emit_kernel(AcceptArgs a) {
+__global__ void __launch_bounds__(ACC_THREADS) accept_emit_kernel(AcceptArgs a, int64_t total) {
     __shared__ int s_scan[ACC_THREADS];
-    const int64_t nbk = n_blocks(a);
-    for (int64_t gblk = blockIdx.x; gblk < nbk; gblk += gridDim.x) {
+    __shared__ int64_t s_block[ACC_THREADS];
+    __shared__ int s_blocks;
+    const int64_t nbk = a.total_blocks_dev ? n_blocks(a) : total;
+    // A CTA's share of the blocks, looked over by a thread each: few blocks
+    // write, and in the FLAG form, whose registers (the FP64 evaluation of the
+    // list's overflow) leave two CTAs on an SM, a CTA per block of a 2^27 cache
+    // spent 91 us on finding that out.
+    const int share = (int)min((int64_t)ACC_THREADS, (nbk + gridDim.x - 1) / gridDim.x);
+    for (int64_t base = blockIdx.x * (int64_t)share; base < nbk;
+         base += (int64_t)gridDim.x * share) {
+    __syncthreads();
+    if (threadIdx.x == 0) s_blocks = 0;
+    __syncthreads();
+    if ((int)threadIdx.x < share && base + threadIdx.x < nbk) {
+        const int64_t g = base + threadIdx.x;
+        const int si = find_seg(a, g);
+        const int64_t boff = a.blk_count[g];
+        // nothing kept in this block: the next block's offset (or the
+        // segment's count) equals this one's
+        const int64_t bnext = g + 1 < seg_base(a, si + 1) ? a.blk_count[g + 1] : a.count[si];
+        if (boff < a.segs[si].max_out && bnext != boff) s_block[atomicAdd(&s_blocks, 1)] = g;
+    }
+    __syncthreads();
+    const int blocks = s_blocks;
+    for (int q = 0; q < blocks; ++q) {
+    const int64_t gblk = s_block[q];
     const int si = find_seg(a, gblk);
     const joker_accept_seg sg = a.segs[si];
     const int64_t blk = gblk - seg_base(a, si);
     const int64_t boff = a.blk_count[gblk];
-    if (boff >= sg.max_out) continue;
-    // nothing kept in this block: the next block's offset (or the segment's
-    // count) equals this one's
-    const int64_t bnext = gblk + 1 < seg_base(a, si + 1) ? a.blk_count[gblk + 1] : a.count[si];
-    if (bnext == boff) continue;
     const uint32_t word = a.words[gblk * ACC_THREADS + threadIdx.x];
     const int c = __popc(word);
     s_scan[threadIdx.x] = c;
@@ -733,6 +730,7 @@ __global__ void __launch_bounds__(ACC_THREADS) accept_emit_kernel(AcceptArgs a) 
         ++pos;
     }
     __syncthreads();
+    }
     }
 }
 
@@ -832,7 +830,7 @@ cudaError_t launch_accept(const AcceptArgs &a, int64_t total_blocks, cudaStream_
 // reads them, so list 1's overflow starts from zero words too.
 cudaError_t launch_accept_fused(const AcceptArgs &a, int64_t total_blocks, cudaStream_t st) {
     if (total_blocks > 0) {
-        const unsigned grid = (unsigned)std::min<int64_t>((total_blocks + 7) / 8, 152 * 8);
+        const unsigned grid = (unsigned)std::min<int64_t>(total_blocks, 152 * 8);
         const size_t wbytes = (size_t)total_blocks * ACC_THREADS * sizeof(uint32_t);
         cudaError_t e = cudaMemsetAsync(a.flag_count, 0, 2 * sizeof(unsigned long long), st);
         if (e == cudaSuccess) e = cudaMemsetAsync(a.amb_words, 0, wbytes, st);
@@ -859,18 +857,19 @@ static cudaError_t accept_finish(const AcceptArgs &a, int64_t total_blocks, cuda
     count_launch();
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || total_blocks == 0) return e;
+    const unsigned emit_grid = (unsigned)std::min<int64_t>(total_blocks, 152 * 8);
     if (a.err != nullptr && a.out_lnl != nullptr) {
         // the ln L written out: FP64 for every output sample with a loose bound
         if ((e = cudaMemsetAsync(a.flag_count, 0, sizeof(unsigned long long), st)) != cudaSuccess)
             return e;
-        accept_emit_kernel<true><<<(unsigned)total_blocks, ACC_THREADS, 0, st>>>(a);
+        accept_emit_kernel<true><<<emit_grid, ACC_THREADS, 0, st>>>(a, total_blocks);
         count_launch();
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         accept_fp64_list_kernel<2><<<152 * 4, 256, 0, st>>>(a, 0, 0);
         count_launch();
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    accept_emit_kernel<false><<<(unsigned)total_blocks, ACC_THREADS, 0, st>>>(a);
+    accept_emit_kernel<false><<<emit_grid, ACC_THREADS, 0, st>>>(a, total_blocks);
     count_launch();
     return cudaGetLastError();
 }
