@@ -24,9 +24,11 @@
 // With the jitter applied the weights change per sample and the full L x L
 // system is factorised per sample (LDL^T, K last).
 //
-// One thread owns one sample and walks the star's epochs, which the CTA
-// stages in shared memory; CTAs pull (star, sample-range) work items from a
-// global counter (a persistent launch sized to the SM count).
+// One thread owns one sample (the FP64 kernel: up to four warps share the
+// epochs of 32 samples) and walks the star's epochs, which the CTA stages in
+// shared memory.  The mixed kernels' CTAs pull (star, sample-range) work items
+// from a global counter (a persistent launch sized to the SM count); the FP64
+// kernel takes one item per CTA.
 #include "joker_mixed.cuh"
 
 namespace joker {
