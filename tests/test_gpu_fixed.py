@@ -128,3 +128,12 @@ def test_period_draws(cuda, lo, hi):
     u = (((c[1] << np.uint64(32)) | c[0]) >> np.uint64(11)).astype(np.float64) * 2.0 ** -53
     want = np.exp(np.log(lo) + u * (np.log(hi) - np.log(lo)))
     np.testing.assert_allclose(P, want, rtol=60 * 2.0 ** -53 * 700)
+
+
+@pytest.mark.parametrize("mean", [np.nan, np.inf, -np.inf])
+def test_prior_mean_not_finite(cuda, mean):
+    """No finite velocity is left: NaN everywhere, as in doubles."""
+    rng = np.random.default_rng(10)
+    star = synth_star(rng, 12, t0=0.0)
+    star["mu"] = np.array([0.0, mean])
+    assert np.all(np.isnan(_lnl(star, synth_chunk(rng, 33), False)))

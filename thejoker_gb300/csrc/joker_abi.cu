@@ -211,6 +211,8 @@ static void prep_fixed(int n, int L, StarRec &r, double *rec64) {
     double tm = 0.0, ym = 0.0, wm = 0.0, wl = INFINITY, Tm[MAXL] = {0.0};
     for (int i = 0; i < n; ++i) {
         const double *q = rec64 + (size_t)i * REC64;
+        // a velocity less a prior mean that is not finite: NaN in doubles
+        if (!std::isfinite(q[0]) || !std::isfinite(q[1])) return;
         tm = std::max(tm, std::fabs(q[0]));
         ym = std::max(ym, std::fabs(q[1]));
         wm = std::max(wm, q[2]);
