@@ -3,12 +3,13 @@
 // One FP64 instruction of a warp holds this GPU's FP64 pipe for 16 cycles of
 // an SM, an FP32 or integer one a quarter of a cycle, so the column and its
 // sums are carried as integers: 62-bit values in two 31-bit limbs, a product
-// three 32 x 32 -> 64 multiply-adds.  FP32 serves where a term is already
-// small (the starter, the first Newton step, the last correction).  Every
-// fixed-point step is good to about 2^-59, the last FP32 correction (of
-// order 2^-31 over f') to 2^-55 over f', f' = 1 - e cos E: below the
-// rounding of the same formulas in doubles, whose phase alone rounds at
-// 2^-53 of the unreduced angle.
+// one 32 x 32 -> 64 multiply and two high halves.  FP32 serves where a term is
+// already small (the starter, the first Newton step, the last correction).
+// Every fixed-point step is good to about 2^-59 whatever the phase; near
+// pericentre the column's error is that over f'^2, f' = 1 - e cos E.  In doubles
+// the same formulas round the phase by 2^-53 of the unreduced angle, over f'^2
+// too, and the rest by 2^-53 over f': as_exact() below is where the first is no
+// larger.
 //
 // Notation: Qn is a real number times 2^n held in an integer.  The eccentric
 // anomaly and the mean anomaly are in turns (Q32, Q63, Q64); a limb pair
@@ -272,6 +273,21 @@ JOKER_FX double exp2_fixed(int n, int64_t f) {
     return double_of(((uint64_t)(1022 + n) << 52) + (uint64_t)((v + 263) >> 9));
 }
 
+// Whether an orbit's column is at least as exact in fixed point as in doubles,
+// for times |dt| 2^tsh < 2^62 whose largest is above half of that: span / P is
+// then above 2^(s-5).  Column errors (rms near pericentre) in fixed point over
+// those in doubles, measured against quadruple precision:
+//   span / P        1 - e = 2^-3..2^-2   2^-6..2^-5   2^-8..2^-7   2^-10..2^-9
+//   1/2 .. 1                  0.27          0.34         0.43          0.70
+//   1/4 .. 1/2                0.43          0.68         0.80          1.4
+//   1/8 .. 1/4                0.59          1.4          1.6           2.7
+//   1/256 .. 1/8              0.42..0.77    2.2..2.9     3.1..9        5..29
+JOKER_FX bool as_exact(int tsh, double P, double e) {
+    const int s = 1088 - tsh - ((int)(bits_of(P) >> 52) & 0x7ff);
+    // by the upper word (a sign or a NaN is Orbit::init's matter): 63/64 and 7/8
+    return s >= 4 || (int32_t)(bits_of(e) >> 32) <= (s == 3 ? 0x3fef8000 : 0x3fec0000);
+}
+
 // One orbit against one star's time scale.
 struct Orbit {
     uint32_t Ri;               // 2^64 turns per unit of the integer epoch times:
@@ -289,9 +305,7 @@ struct Orbit {
 
     // Integer times are t = dt 2^tsh - t0.  False: outside the fixed-point
     // form's range, whose lines are the phase's 2^32 turns per time scale,
-    // angles below 2^10, and e <= 0.999, to where the fixed-point form is at
-    // least as exact as the FP64 one (its last FP32 correction grows as
-    // 1 / f'^2 beyond).
+    // angles below 2^10, and e <= 0.999 (see as_exact for its exactness).
     JOKER_FX bool init(int tsh, int64_t t0, double P, double e_, double om, double M0) {
         far_r = 0;
         far_d = 0.0f;

@@ -302,7 +302,8 @@ struct AccFx {
             g = rcp_newton(1.0 + a);
             g62 = fx::split(fx::fixed62(g));
         }
-        return st.fx_ok && orb.init(st.fx_tsh, st.fx_t0, P, e, om, M0);
+        return st.fx_ok && fx::as_exact(st.fx_tsh, P, e) &&
+               orb.init(st.fx_tsh, st.fx_t0, P, e, om, M0);
     }
 
     __device__ __forceinline__ void add(const fx::EpochFx &r) {

@@ -378,6 +378,7 @@ rv_elements_kernel(const double *t, int n_t, const double *el, int64_t n, int pe
         const int tsh = 62 - ((int)ex - 1022);            // |dt| 2^tsh < 2^62
         fx::Orbit orb;
         bool ok = ex > 723 && ex < 1323 &&                // within 2^300 of one day
+                  fx::as_exact(tsh, p[0], p[2]) &&
                   orb.init(tsh, -fx::ONE62, p[0], p[2], p[3], p[4]);
         if (ok) {
             for (int j = lane; j < nt; j += 32) {
