@@ -181,7 +181,9 @@ posterior_kernel(const StarRec *stars, const double *ep64, int star, const doubl
     const int64_t r = rows[active ? i : n - 1] * stride;
     const double p = P[r], e = E[r], om = OM[r], m0 = M0[r], s = JIT ? S[r] : 0.0;
     AccFx<L, JIT> acc;
-    bool ok = acc.init(st, p, e, om, m0, s);
+    // mu0 as the device has it: a launch captured for one star of a slot may be
+    // replayed for another
+    bool ok = st.mu0 == 0.0 && acc.init(st, p, e, om, m0, s);
     if (!sliced_epochs(acc, active && ok, st, ep64, smem, slices) || !active) return;
     double *a_out = a + i * L, *A_out = A + i * L * L, *l_out = lnl ? lnl + i : nullptr;
     if (!ok || acc.orb.bad()) {
