@@ -125,9 +125,11 @@ __device__ __forceinline__ void posterior_schur(const StarRec &st, double A00, c
         gv = fma(A0[j], v[j], gv);
         u = fma(-A0[j], st.cC[j], u);
     }
-    const double ls = fma(lam0, A00 - gv, 1.0);               // Lambda0 s
+    const double sm = A00 - gv, ls = fma(lam0, sm, 1.0);      // Lambda0 s
     const bool ok = ls > 0.0;
-    const double is = lam0 * (ls < 1e300 ? rcp_newton(ls) : 1.0 / ls);
+    // (Lambda0 s beyond a double's range, or Lambda0 infinite: 1/s by itself)
+    const bool big = !(ls < 1e300);
+    const double is = big ? 1.0 / (sm + 1.0 / lam0) : lam0 * rcp_newton(ls);
     const double K = u * is;
     a_out[0] = ok ? K : NAN;
     A_out[0] = ok ? is : NAN;
@@ -141,7 +143,8 @@ __device__ __forceinline__ void posterior_schur(const StarRec &st, double A00, c
             A_out[j * L + k] = A_out[k * L + j] = ok ? fma(w, v[k], st.Cinv[j * MAXL + k]) : NAN;
     }
     if (lnl_out)
-        *lnl_out = ok ? -0.5 * (fma(-u, K, st.chi2_0) + st.logdet_const + log(ls)) : INFINITY;
+        *lnl_out = ok ? -0.5 * (fma(-u, K, st.chi2_0) + st.logdet_const +
+                                (big ? log(lam0) - log(is) : log(ls))) : INFINITY;
 }
 
 // In doubles, one thread: the form for what the fixed-point one does not take.
