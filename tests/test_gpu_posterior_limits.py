@@ -65,3 +65,17 @@ def test_wide_prior(cuda, lam0, poly, jitter):
         assert np.all(np.abs(lnl - el) <= 1e-9 * grow * np.maximum(1.0, np.abs(el)))
     else:
         assert np.all(lnl == -np.inf)
+
+
+@pytest.mark.parametrize("jitter", [False, True])
+@pytest.mark.parametrize("N,poly", [(3, 1), (20, 2), (40, 1)])
+def test_parabolic_row(cuda, N, poly, jitter):
+    """e = 1: an infinite K prior variance; the unit-K column is the limit's, and
+    the row is finite."""
+    rng = np.random.default_rng(N)
+    star = synth_star(rng, N, poly=poly, t0=0.0, base=100.0)
+    chunk = synth_chunk(rng, 5, P_max=60.0, jitter=jitter)
+    chunk[2, 1] = 1.0
+    a, A, lnl = _posterior(star, chunk, jitter)
+    assert np.all(np.isfinite(a)) and np.all(np.isfinite(A))
+    assert lnl[2] == -np.inf and np.all(np.isfinite(np.delete(lnl, 2)))

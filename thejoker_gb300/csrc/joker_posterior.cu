@@ -161,8 +161,13 @@ __device__ __noinline__ void posterior_doubles(const StarRec &st, const double *
         for (int k = 1; k < L; ++k) T[k - 1] = __ldg(rec + 2 + k);
         acc.add(__ldg(rec), __ldg(rec + 1), __ldg(rec + 2), T);
     }
+    double lam0 = k_prior_variance(st, P, e, k_clip != 0);
+    if (st.k_scaled && e * e == 1.0) {                        // no reciprocal of zero
+        lam0 = st.sigK0sq / (1.0 - e * e) * pow(P / st.P0, -2.0 / 3.0);
+        if (k_clip) lam0 = fmin(st.maxK2, lam0);
+    }
     posterior_tail<L>(st, acc.G, acc.q, acc.rWr, st.log_norm_rest - acc.sum_log_w(st), LogProd(),
-                      k_prior_variance(st, P, e, k_clip != 0), a_out, A_out, lnl_out);
+                      lam0, a_out, A_out, lnl_out);
 }
 
 // One sample per thread, epochs shared out over S warps (sliced_epochs).
