@@ -361,59 +361,75 @@ __global__ void __launch_bounds__(256) unmarginalized_kernel(const StarRec *star
 }
 
 // rv[i * n_t + j] = K_i m_i(t_j - t0) for element rows (P, K, e, omega, M0).
-// A warp takes RV_TIMES times of one orbit, so that the orbit's constants are
-// made once for them; the times become integers on the scale of the largest.
-// One thread per (orbit, time) pair made them for each pair, and in doubles:
-// 4096 orbits x 1001 times took 785 us.
-constexpr int RV_LANE = 8, RV_TIMES = 32 * RV_LANE;
+// W lanes take up to 8 W times of one orbit, so that the orbit's constants are
+// made once a lane for them; the times become integers on the scale of the
+// largest.  One thread per (orbit, time) pair made them for each pair, and in
+// doubles: 4096 orbits x 1001 times took 785 us, now 82 (W = 32).
+constexpr int RV_LANE = 8;
 
+template <int W>
 __global__ void __launch_bounds__(128, 6)
 rv_elements_kernel(const double *t, int n_t, const double *el, int64_t n, int per_row, double t0,
                    double *rv) {
-    const int lane = threadIdx.x & 31;
-    const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t g = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
-         g < n * per_row; g += nw) {
+    const int lane = threadIdx.x & (W - 1);
+    // the group's lanes; groups of a warp go their own ways
+    const unsigned group = W == 32 ? 0xffffffffu
+                                   : ((1u << W % 32) - 1u) << (threadIdx.x & 31 & ~(W - 1));
+    const int64_t step = (int64_t)gridDim.x * (blockDim.x / W);
+    for (int64_t g = blockIdx.x * (int64_t)(blockDim.x / W) + threadIdx.x / W; g < n * per_row;
+         g += step) {
         const int64_t i = g / per_row;
-        const int j0 = (int)(g - i * per_row) * RV_TIMES;
-        const int nt = min(n_t - j0, RV_TIMES);
+        const int j0 = (int)(g - i * per_row) * (W * RV_LANE);
+        const int nt = min(n_t - j0, W * RV_LANE);
         const double *p = el + i * 5;
         const double K = p[1];
         double *out = rv + i * n_t + j0;
         // the exponent of the largest |dt|: 2^(ex - 1023) <= |dt| < twice that
         unsigned ex = 0;
-        for (int j = lane; j < nt; j += 32)
+        for (int j = lane; j < nt; j += W)
             ex = max(ex, (unsigned)(__double2hiint(t[j0 + j] - t0) >> 20) & 0x7ff);
-        ex = __reduce_max_sync(0xffffffffu, ex);
+        if (W > 1) ex = __reduce_max_sync(group, ex);
         const int tsh = 62 - ((int)ex - 1022);            // |dt| 2^tsh < 2^62
         fx::Orbit orb;
         bool ok = ex > 723 && ex < 1323 &&                // within 2^300 of one day
                   fx::as_exact(tsh, p[0], p[2]) &&
                   orb.init(tsh, -fx::ONE62, p[0], p[2], p[3], p[4]);
         if (ok) {
-            for (int j = lane; j < nt; j += 32) {
+            for (int j = lane; j < nt; j += W) {
                 const int64_t q = fx::fixed_signed(t[j0 + j] - t0, tsh);
                 const double m = (double)orb.column((uint64_t)(q + fx::ONE62));
                 out[j] = K * (m * 0x1p-61);
             }
-            ok = !__any_sync(0xffffffffu, orb.bad());
+            ok = W > 1 ? !__any_sync(group, orb.bad()) : !orb.bad();
         }
         if (!ok) {
             OrbitF64 o;
             o.init(p[0], p[2], p[3], p[4]);
-            for (int j = lane; j < nt; j += 32) out[j] = K * o.rv_unit(t[j0 + j] - t0);
+            for (int j = lane; j < nt; j += W) out[j] = K * o.rv_unit(t[j0 + j] - t0);
         }
     }
 }
 
-cudaError_t launch_rv_elements(const double *t, int n_t, const double *el, int64_t n, double t0,
-                               double *rv, cudaStream_t st) {
-    const int per_row = (n_t + RV_TIMES - 1) / RV_TIMES;
-    const int64_t blocks = (n * per_row + 3) / 4;
+template <int W>
+static cudaError_t launch_rv(const double *t, int n_t, const double *el, int64_t n, double t0,
+                             double *rv, cudaStream_t st) {
+    const int per_row = (n_t + W * RV_LANE - 1) / (W * RV_LANE), groups = 128 / W;
+    const int64_t blocks = (n * per_row + groups - 1) / groups;
     const unsigned grid = (unsigned)(blocks < 152 * 64 ? blocks : 152 * 64);
-    rv_elements_kernel<<<grid, 128, 0, st>>>(t, n_t, el, n, per_row, t0, rv);
+    rv_elements_kernel<W><<<grid, 128, 0, st>>>(t, n_t, el, n, per_row, t0, rv);
     count_launch();
     return cudaGetLastError();
+}
+
+// Lanes per orbit: a lane without a time still makes the orbit's constants (450
+// instructions against a column's 250), so curves of a few times take fewer.
+// 10^6 orbits x 1 time: a thread per pair in doubles 196 us, 32 lanes 1085, one
+// 40; x 7 times: 1340, 1084, eight lanes 291; x 9: 1717, 1096 (32 lanes).
+cudaError_t launch_rv_elements(const double *t, int n_t, const double *el, int64_t n, double t0,
+                               double *rv, cudaStream_t st) {
+    if (n_t == 1) return launch_rv<1>(t, n_t, el, n, t0, rv, st);
+    if (n_t <= 8) return launch_rv<8>(t, n_t, el, n, t0, rv, st);
+    return launch_rv<32>(t, n_t, el, n, t0, rv, st);
 }
 
 template <int L, bool JIT>
