@@ -56,7 +56,7 @@ struct joker_stars {
     int slot_epochs = 0;         // > 0 for a slot table (joker_stars_create_slots)
     int64_t total_epochs = 0;
     std::vector<int64_t> off;
-    std::vector<unsigned char> fixed;   // per star: see stars_fixed
+    std::vector<unsigned char> fixed;   // per star: 1 fixed-point form, 2 and K's mean is 0
     StarRec *d_stars = nullptr;
     double *d_ep64 = nullptr;
     float *d_ep32 = nullptr;
@@ -253,6 +253,10 @@ static void prep_fixed(int n, int L, StarRec &r, double *rec64) {
         memcpy(q + FX64, &f, sizeof f);
     }
     r.fx_ok = 1;
+}
+
+static unsigned char fixed_flags(const StarRec &r) {
+    return r.fx_ok ? (r.mu0 == 0.0 ? 3 : 1) : 0;
 }
 
 // Per-star preparation on the host, in FP64 / long double: the StarRec
@@ -540,7 +544,7 @@ extern "C" int joker_stars_create(joker_stars **out, int n_stars, int n_linear,
     s->total_epochs = NE;
     s->off.assign(epoch_offsets, epoch_offsets + n_stars + 1);
     for (int k = 0; k < n_stars; ++k)
-        s->fixed.push_back(recs[k].fx_ok && recs[k].mu0 == 0.0);
+        s->fixed.push_back(fixed_flags(recs[k]));
     cudaError_t e = parts.allocate(s);
     if (e != cudaSuccess) {
         joker_stars_destroy(s);
@@ -628,7 +632,7 @@ extern "C" int joker_stars_set(joker_stars *s, int slot, int n_epochs, const dou
     CUDA_TRY(cudaMemcpyAsync(s->d_ep32 + (size_t)r.epoch_off * REC32, r32.data(),
                              sizeof(float) * r32.size(), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(s->d_stars + slot, &r, sizeof(StarRec), cudaMemcpyHostToDevice, st));
-    s->fixed[slot] = r.fx_ok && r.mu0 == 0.0;
+    s->fixed[slot] = fixed_flags(r);
     // pageable sources: staged before the calls return
     return JOKER_OK;
 }
@@ -829,6 +833,11 @@ static int run_lnl(const joker_stars *s, int precision, LnlArgs a, int block,
     // the FP64 kernel takes its items by block
     if (precision != JOKER_FP64) CUDA_TRY(cudaMemsetAsync(s->d_queue, 0, sizeof(int), st));
     a.max_epochs = s->max_epochs;
+    // (a launch captured for other stars is right either way: both kernels take
+    // what the record lacks or has from the device)
+    a.doubles = 1;
+    for (int k = a.star0; k < a.star0 + a.n_sel && a.doubles; ++k)
+        a.doubles = !(s->fixed[k] & (s->jitter == JOKER_JITTER_APPLIED ? 2 : 1));
     CUDA_TRY(launch_lnl(precision, s->L, s->jitter == JOKER_JITTER_APPLIED, a, block, st));
     return JOKER_OK;
 }
@@ -881,7 +890,7 @@ void stars_internals(const joker_stars *s, const StarRec **recs, const double **
 int stars_max_epochs(const joker_stars *s) { return s->max_epochs; }
 // whether the star's records have the fixed-point form and its K prior mean is
 // zero, as that form's full system wants
-bool stars_fixed(const joker_stars *s, int star) { return s->fixed[star] != 0; }
+bool stars_fixed(const joker_stars *s, int star) { return (s->fixed[star] & 2) != 0; }
 
 void cache_internals(const joker_cache *c, int64_t *cap, const double **P, const double **E,
                      const double **OM, const double **M0, const double **S, int64_t *stride,

@@ -114,6 +114,7 @@ struct LnlArgs {
     const int *n_items_dev;  // when set, the item count is read from device memory
     int star0, n_sel, chunk;
     int max_epochs;          // of the table
+    int doubles;             // FP64, implicit items: no star has the fixed-point form
     int64_t row0, count, ld, ips;
     const int *order;
     int *queue;              // dynamic work counter, zeroed before launch

@@ -72,6 +72,53 @@ lnl_fp64_kernel(LnlArgs a, int S) {
     }
 }
 
+// The same for calls none of whose stars has the fixed-point form (weights more
+// than 2^8 apart, or with the jitter a K prior mean), one sample per thread in
+// doubles: FP64 pipe, 70-90 instructions an epoch.  Through the kernel above
+// such calls carried its state beside theirs, and under S = 4 one warp of four
+// worked: 2^20 samples x 16 epochs 2308 us, here 2179, with the jitter 2731 and
+// 2586; 60013 x 40 341 and 323.
+template <int L, bool JIT>
+__global__ void __launch_bounds__(SLICED_BLOCK) lnl_fp64_doubles_kernel(LnlArgs a) {
+    __shared__ __align__(16) double sm[TILE * FX64];
+    const int n_items = item_count(a);
+    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
+        const WorkItem w = get_item(a, it);
+        const StarRec &st = a.stars[w.star];
+        const int N = st.n_epochs;
+        unsigned long long *mk = a.max_key ? a.max_key + w.max_slot : nullptr;
+        for (int base = 0; base < w.count; base += blockDim.x) {
+            const int j = base + threadIdx.x;
+            const bool active = j < w.count;
+            const int64_t row = (w.row0 + (active ? j : 0)) * a.stride;
+            const double P = a.P[row];
+            Acc64<L, JIT> acc;
+            acc.init(st, P, a.e[row], a.om[row], a.M0[row], JIT ? a.s[row] : 0.0);
+            for (int t0 = 0; t0 < N; t0 += TILE) {
+                const int nt = min(TILE, N - t0);
+                const double2 *src = reinterpret_cast<const double2 *>(
+                    a.ep64 + ((size_t)st.epoch_off + t0) * REC64);
+                __syncthreads();
+                for (int i = threadIdx.x; i < nt * (FX64 / 2); i += blockDim.x)
+                    reinterpret_cast<double2 *>(sm)[i] =
+                        __ldg(src + i / (FX64 / 2) * (REC64 / 2) + i % (FX64 / 2));
+                __syncthreads();
+                if (active)
+                    for (int i = 0; i < nt; ++i) {
+                        const double *rec = sm + i * FX64;
+                        acc.add(rec[0], rec[1], rec[2], rec + 3);
+                    }
+            }
+            double lnl = 0.0;
+            if (active) {
+                lnl = acc.finish(st, P);
+                a.lnl[w.out_off + j] = lnl;
+            }
+            if (mk) warp_max_update(mk, active ? double_to_key(lnl) : 0ull);
+        }
+    }
+}
+
 // --------------------------------------------------------- cache preparation
 // From the reference's packed chunk (n x 5 row-major FP64: P, e, omega, M0, s)
 // to FP64 columns and the prepared mixed form.
@@ -102,14 +149,20 @@ cudaError_t launch_lnl_packed(int precision, int L, bool jit, const LnlArgs &a, 
 // a count in device memory is shared out over a grid of one wave.
 template <int L, bool JIT>
 static cudaError_t launch_fp64_LJ(LnlArgs a, cudaStream_t st) {
-    int grid = a.n_items, S = 1;
+    int grid = a.n_items, S = 1, block = SLICED_BLOCK;
     if (a.n_items_dev) {
         const cudaError_t e = persistent_grid(
             reinterpret_cast<const void *>(lnl_fp64_kernel<L, JIT>), SLICED_BLOCK, &grid);
         if (e != cudaSuccess) return e;
     } else if (!a.items) {
-        S = slices_for(a.count * a.n_sel, a.max_epochs);
-        const int64_t chunk = SLICED_BLOCK / S, ips = (a.count + chunk - 1) / chunk;
+        // doubles: blocks of a warp while blocks of four would leave the SMs'
+        // shares uneven (60013 x 40: 383 -> 323 us; 200000 x 40: 1046 -> 1017;
+        // 310000 x 16: 652 -> 663)
+        if (a.doubles)
+            block = a.count * a.n_sel < 12 * 152 * SLICED_BLOCK ? 32 : SLICED_BLOCK;
+        else
+            S = slices_for(a.count * a.n_sel, a.max_epochs);
+        const int64_t chunk = block / S, ips = (a.count + chunk - 1) / chunk;
         if (ips * a.n_sel <= INT32_MAX) {
             a.chunk = (int)chunk;
             a.ips = ips;
@@ -117,7 +170,10 @@ static cudaError_t launch_fp64_LJ(LnlArgs a, cudaStream_t st) {
         }
     }
     if (grid < 1) return cudaSuccess;
-    lnl_fp64_kernel<L, JIT><<<grid, SLICED_BLOCK, sliced_smem<L, JIT>(S), st>>>(a, S);
+    if (a.doubles)
+        lnl_fp64_doubles_kernel<L, JIT><<<grid, block, 0, st>>>(a);
+    else
+        lnl_fp64_kernel<L, JIT><<<grid, SLICED_BLOCK, sliced_smem<L, JIT>(S), st>>>(a, S);
     count_launch();
     return cudaGetLastError();
 }
