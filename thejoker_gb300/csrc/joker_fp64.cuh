@@ -262,9 +262,25 @@ __device__ __forceinline__ double Acc64<L, JIT>::finish(const StarRec &st, doubl
     }
 }
 
+// A product of numbers in (0, 1], m 2^(e - 62) with m in [2^61, 2^62).  Each
+// factor truncates it, so its last bits depend on the factors' order.
+struct FxProd {
+    int64_t m;
+    int32_t e;
+    __device__ __forceinline__ void one() { m = fx::ONE62 - 1; e = 0; }
+    __device__ __forceinline__ void times(int64_t m2, int32_t e2 = 0) {
+        m = fx::mul(fx::split(m), fx::split(m2));
+        const int z = fx::clz64((uint64_t)m) - 2;
+        m <<= z;
+        e += e2 - z;
+    }
+};
+
 // Per-sample state of the fixed-point form: the integer epoch sums, and the
 // same finish as Acc64's from their doubles.  Sums of integers do not depend
-// on the order, so every split of the epochs over threads gives the same ln L.
+// on the order; the jitter's product is kept as four, of epochs i with the same
+// i mod 4 in their order, that meet in that of i mod 4.  So every split of the
+// epochs over threads gives the same ln L.
 //
 // With the jitter the weights are w_j = 2^ew g wn_j, g = 1 / (1 + a),
 // a = s^2 2^ew, wn_j = v_j / d_j, v_j = ivar_j 2^-ew and
@@ -277,8 +293,7 @@ struct AccFx {
     fx::Sum96 G[L][L], q[L], rWr;            // jitter: the rest
     fx::limbs g62;
     double g, a;
-    int64_t pj;                              // prod d_j = pj 2^(ej - 62)
-    int ej;
+    FxProd prod;                             // of the d_j, set before finish
 
     // False: the sample (or star) needs the FP64 form.
     __device__ __forceinline__ bool init(const StarRec &st, double P, double e, double om,
@@ -295,8 +310,6 @@ struct AccFx {
                 for (int k = 0; k < L; ++k) G[i][k].zero();
             }
             rWr.zero();
-            pj = fx::ONE62 - 1;
-            ej = 0;
             a = s * s * st.fx_w;
             if (!(st.mu0 == 0.0 && a <= 0x1p40)) return false;
             g = rcp_newton(1.0 + a);
@@ -306,7 +319,8 @@ struct AccFx {
                orb.init(st.fx_tsh, st.fx_t0, P, e, om, M0);
     }
 
-    __device__ __forceinline__ void add(const fx::EpochFx &r) {
+    // One epoch; with the jitter, its d_j (Q62).
+    __device__ __forceinline__ int64_t add(const fx::EpochFx &r) {
         const int64_t mq = orb.column(r.t);                            // Q61
         const fx::limbs m = fx::split(mq);
         if (!JIT) {
@@ -317,11 +331,11 @@ struct AccFx {
             if (L > 1) A0[1].add(wmq);                                 // Q61; T_1 = 1
 #pragma unroll
             for (int k = 2; k < L; ++k) A0[k].add(fx::mul(wm, r.T[k - 2]));
+            return 0;
         } else {
             const int64_t v = fx::join(r.w);
             const int64_t d = fx::clamp62(v + fx::mul(g62, fx::split(fx::ONE62 - v)));
             const int64_t wq = fx::twice(fx::div61(v >> 1, d >> 1));   // Q62
-            times(d, 0);
             const fx::limbs w = fx::split(wq);
             const int64_t wmq = fx::mul(w, m), wyq = fx::mul(w, r.y);
             const fx::limbs wm = fx::split(wmq), wy = fx::split(wyq);
@@ -343,6 +357,7 @@ struct AccFx {
 #pragma unroll
                 for (int k = 2; k <= i; ++k) G[i][k].add(fx::mul(wT, r.T[k - 2]));
             }
+            return d;
         }
     }
 
@@ -363,28 +378,14 @@ struct AccFx {
         }
     }
     static constexpr int SUMS = 1 + L + (JIT ? L + L * (L - 1) / 2 : 0);
-    static constexpr int WORDS = 3 * SUMS + 1 + (JIT ? 3 : 0);           // of a stored state
+    static constexpr int WORDS = 3 * SUMS + 1 + (JIT ? 1 : 0);           // of a stored state
 
-    __device__ __forceinline__ void times(int64_t p2, int e2) {
-        pj = fx::mul(fx::split(pj), fx::split(p2));
-        const int z = fx::clz64((uint64_t)pj) - 2;
-        pj <<= z;
-        ej += e2 - z;
-    }
-
-    // Over the 32 lanes of a warp (every lane gets the totals).
+    // The sums over the 32 lanes of a warp (every lane gets the totals).
     __device__ __forceinline__ void warp_sum() {
         each([](fx::Sum96 &v) { v.warp_sum(); });
-        if (JIT) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const int64_t p2 = (int64_t)__shfl_xor_sync(0xffffffffu, (unsigned long long)pj, o);
-                times(p2, __shfl_xor_sync(0xffffffffu, ej, o));
-            }
-        }
     }
 
-    // The sums as WORDS words, 32 apart, and the sum with such a state.
+    // The sums (and prod's e) as WORDS words, 32 apart, and the sum with such a state.
     __device__ __forceinline__ void store(uint32_t *w) {
         int k = 0;
         auto put = [&](uint32_t v) { w[32 * k++] = v; };
@@ -394,11 +395,7 @@ struct AccFx {
             put((uint32_t)v.hi);
         });
         put(orb.bad());
-        if (JIT) {
-            put((uint32_t)pj);
-            put((uint32_t)((uint64_t)pj >> 32));
-            put((uint32_t)ej);
-        }
+        if (JIT) put((uint32_t)prod.e);
     }
     __device__ __forceinline__ void merge(const uint32_t *w) {
         int k = 0;
@@ -412,10 +409,7 @@ struct AccFx {
             v.add(l, (int32_t)get());
         });
         if (get()) orb.far_r = fx::RI_MAX + 1;
-        if (JIT) {
-            const int64_t p2 = (int64_t)get64();
-            times(p2, (int32_t)get());
-        }
+        if (JIT) prod.e += (int32_t)get();
     }
 
     // The jitter form's sums as doubles: the lower triangle of M W M^T, M W y
@@ -449,8 +443,8 @@ struct AccFx {
 
     // sum log(1 + s^2 ivar_j) less log of the returned factor in [1/2, 1)
     __device__ __forceinline__ double log_rest(const StarRec &st, double &factor) const {
-        factor = (double)pj * 0x1p-62;
-        return fma((double)ej, 0.69314718055994530942, (double)st.n_epochs * log1p(a));
+        factor = (double)prod.m * 0x1p-62;
+        return fma((double)prod.e, 0.69314718055994530942, (double)st.n_epochs * log1p(a));
     }
 
     __device__ __forceinline__ double finish(const StarRec &st, double P, double e) const {
@@ -502,11 +496,15 @@ constexpr int SLICED_BLOCK = 128;
 // the jitter form would spill their sums.
 constexpr int fx_blocks(int L, bool jit) { return jit && L > 3 ? 3 : 6; }
 
-// Shared memory of such a block: a tile of epochs, then the stored states.
-template <int L, bool JIT> constexpr int sliced_smem(int S) {
+// Shared memory of such a block: a tile of epochs, then the stored states; with
+// the jitter, behind them, the four products of each sample.
+template <int L, bool JIT> __host__ __device__ constexpr int sliced_states(int S) {
     const int tile = TILE * (int)sizeof(fx::EpochFx);
     const int states = (4 / S) * (S - 1) * AccFx<L, JIT>::WORDS * 128;
     return tile > states ? tile : states;
+}
+template <int L, bool JIT> constexpr int sliced_smem(int S) {
+    return sliced_states<L, JIT>(S) + (JIT ? 4 * (SLICED_BLOCK / S) * 8 : 0);
 }
 
 // All epochs of a star into the samples' states; afterwards the first warp of
@@ -517,23 +515,46 @@ __device__ __forceinline__ bool sliced_epochs(AccFx<L, JIT> &acc, bool go, const
                                               const double *ep64, void *smem, int S) {
     fx::EpochFx *sm = static_cast<fx::EpochFx *>(smem);
     const int warp = threadIdx.x >> 5, slice = warp & (S - 1), N = st.n_epochs;
+    // m of product c of this thread's sample at c * samples (their e's add up)
+    const int samples = SLICED_BLOCK / S;
+    int64_t *pm = reinterpret_cast<int64_t *>(static_cast<char *>(smem) +
+                                              sliced_states<L, JIT>(S)) +
+                  warp / S * 32 + (threadIdx.x & 31);
+    if (JIT) {
+        if (S > 1) __syncthreads();              // an earlier call's products are read
+        acc.prod.one();
+        for (int c = slice; c < 4; c += S) pm[c * samples] = acc.prod.m;
+    }
     for (int t0 = 0; t0 < N; t0 += TILE) {
         const int nt = min(TILE, N - t0);
         __syncthreads();
         stage_epochs_fx(sm, ep64 + ((size_t)st.epoch_off + t0) * REC64, nt);
         __syncthreads();
         if (go)
-            for (int i = (slice - t0) & (S - 1); i < nt; i += S) acc.add(sm[i]);
+            for (int i = (slice - t0) & (S - 1); i < nt; i += S) {
+                const int64_t d = acc.add(sm[i]);
+                if (JIT) {
+                    int64_t *m = pm + (i & 3) * samples;         // TILE is a multiple of 4
+                    acc.prod.m = *m;
+                    acc.prod.times(d);
+                    *m = acc.prod.m;
+                }
+            }
     }
-    if (S == 1) return true;
-    __syncthreads();
-    uint32_t *w = static_cast<uint32_t *>(smem) +
-                  ((warp / S) * (S - 1) * AccFx<L, JIT>::WORDS) * 32 + (threadIdx.x & 31);
-    if (slice > 0) acc.store(w + (slice - 1) * AccFx<L, JIT>::WORDS * 32);
-    __syncthreads();
-    if (slice == 0)
+    if (S > 1) {
+        __syncthreads();
+        uint32_t *w = static_cast<uint32_t *>(smem) +
+                      ((warp / S) * (S - 1) * AccFx<L, JIT>::WORDS) * 32 + (threadIdx.x & 31);
+        if (slice > 0) acc.store(w + (slice - 1) * AccFx<L, JIT>::WORDS * 32);
+        __syncthreads();
+        if (slice > 0) return false;
         for (int k = 0; k < S - 1; ++k) acc.merge(w + k * AccFx<L, JIT>::WORDS * 32);
-    return slice == 0;
+    }
+    if (JIT) {
+        acc.prod.m = pm[0];
+        for (int c = 1; c < 4; ++c) acc.prod.times(pm[c * samples]);
+    }
+    return true;
 }
 
 // S for n samples of at most N epochs: four while the 128-sample blocks would
@@ -567,7 +588,15 @@ __device__ __noinline__ double fp64_lnl_global(const StarRec &st, const double *
     AccFx<L, JIT> acc;
     if (acc.init(st, P, e, om, M0, s)) {
         const double *rec = ep64 + (size_t)st.epoch_off * REC64;
-        for (int i = 0; i < st.n_epochs; ++i, rec += REC64) acc.add(load_epoch_fx(rec));
+        FxProd p[4];
+        for (int c = 0; c < 4; ++c) p[c].one();
+        for (int i = 0; i < st.n_epochs; ++i, rec += REC64) {
+            const int64_t d = acc.add(load_epoch_fx(rec));
+            if (JIT) p[i & 3].times(d);
+        }
+        acc.prod = p[0];
+        if (JIT)
+            for (int c = 1; c < 4; ++c) acc.prod.times(p[c].m, p[c].e);
         if (!acc.orb.bad()) return acc.finish(st, P, e);
     }
     return fp64_lnl_doubles<L, JIT>(st, ep64, P, e, om, M0, s);
@@ -584,9 +613,28 @@ __device__ __noinline__ double fp64_lnl_warp_t(const StarRec &st, const double *
     const double *rec0 = ep64 + (size_t)st.epoch_off * REC64;
     AccFx<L, JIT> fxa;
     if (fxa.init(st, P, e, om, M0, s)) {
-        for (int i = threadIdx.x & 31; i < st.n_epochs; i += 32)
-            fxa.add(load_epoch_fx(rec0 + (size_t)i * REC64));
+        const int lane = threadIdx.x & 31;
+        FxProd p;                                // that of epochs i = lane mod 4
+        p.one();
+        for (int base = 0; base < st.n_epochs; base += 32) {
+            int64_t d = 0;
+            if (base + lane < st.n_epochs)
+                d = fxa.add(load_epoch_fx(rec0 + (size_t)(base + lane) * REC64));
+            if (JIT)
+                for (int k = lane & 3, n = 0; n < 8; k += 4, ++n) {
+                    const int64_t dk =
+                        (int64_t)__shfl_sync(0xffffffffu, (unsigned long long)d, k);
+                    if (base + k < st.n_epochs) p.times(dk);
+                }
+        }
         fxa.warp_sum();
+        if (JIT) {
+            fxa.prod.m = (int64_t)__shfl_sync(0xffffffffu, (unsigned long long)p.m, 0);
+            fxa.prod.e = __shfl_sync(0xffffffffu, p.e, 0);
+            for (int c = 1; c < 4; ++c)
+                fxa.prod.times((int64_t)__shfl_sync(0xffffffffu, (unsigned long long)p.m, c),
+                               __shfl_sync(0xffffffffu, p.e, c));
+        }
         if (!__any_sync(0xffffffffu, fxa.orb.bad())) return fxa.finish(st, P, e);
     }
     Acc64<L, JIT> acc;

@@ -38,7 +38,7 @@ namespace joker {
 // it does not take runs in doubles (fp64_lnl_doubles).  In doubles the FP64
 // pipe bounded it (70-90 FP64 instructions per epoch, 16 cycles of an SM
 // each); in fixed point the integer pipes do.  2^20 samples x 16 epochs:
-// 2267 us in doubles, 318 us; 1.5e6 x 40 with the jitter: 9041, 1377 us.
+// 2267 us in doubles, 318 us; 1.5e6 x 40 with the jitter: 9041, 1403 us.
 // What bounds it now is the pipe of the wide integer multiplies (73 % busy).
 template <int L, bool JIT>
 __global__ void __launch_bounds__(SLICED_BLOCK, fx_blocks(L, JIT))
