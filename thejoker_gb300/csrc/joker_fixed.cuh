@@ -203,11 +203,11 @@ JOKER_FX uint64_t shift(uint64_t v, int k) {
 }
 JOKER_FX int64_t clamp62(int64_t v) { return v > ONE62 - 1 ? ONE62 - 1 : v; }
 JOKER_FX int64_t twice(int64_t v) { return clamp62(v + v); }
-// x in [0, 1] as Q62, at most 1 - 2^-62
+// x in [0, 1] (-0 too) as Q62, at most 1 - 2^-62
 JOKER_FX int64_t fixed62(double x) {
     const uint64_t b = bits_of(x);
     return clamp62((int64_t)shift((b & 0xfffffffffffffull) | 0x10000000000000ull,
-                                  (int)(b >> 52) - 1013));
+                                  ((int)(b >> 52) & 0x7ff) - 1013));
 }
 // x 2^q, the bits below the unit dropped, for |x| 2^q < 2^63
 JOKER_FX int64_t fixed_signed(double x, int q) {
