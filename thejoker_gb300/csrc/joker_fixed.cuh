@@ -303,12 +303,14 @@ struct Orbit {
     int32_t far_r;             // the largest |ri| and |dl| of the columns so far
     float far_d;
 
+    // No column yet; what bad() reads of an orbit that init refused or never saw.
+    JOKER_FX void clear() { far_r = 0; far_d = cs = 0.0f; }
+
     // Integer times are t = dt 2^tsh - t0.  False: outside the fixed-point
     // form's range, whose lines are the phase's 2^32 turns per time scale,
     // angles below 2^10, and e <= 0.999 (see as_exact for its exactness).
     JOKER_FX bool init(int tsh, int64_t t0, double P, double e_, double om, double M0) {
-        far_r = 0;
-        far_d = 0.0f;
+        clear();
         const uint64_t pb = bits_of(P);
         const int pe = (int)(pb >> 52);                       // sign bit too
         const int s = 1088 - tsh - pe;

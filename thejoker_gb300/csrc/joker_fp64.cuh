@@ -298,6 +298,7 @@ struct AccFx {
     // False: the sample (or star) needs the FP64 form.
     __device__ __forceinline__ bool init(const StarRec &st, double P, double e, double om,
                                          double M0, double s) {
+        orb.clear();                             // sliced_epochs stores bad() of every sample
         A00.zero();
         b0.zero();
 #pragma unroll
