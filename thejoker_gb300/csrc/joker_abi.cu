@@ -56,6 +56,7 @@ struct joker_stars {
     int slot_epochs = 0;         // > 0 for a slot table (joker_stars_create_slots)
     int64_t total_epochs = 0;
     std::vector<int64_t> off;
+    std::vector<int> epochs;            // per star; 0: an empty slot
     std::vector<unsigned char> fixed;   // per star: 1 fixed-point form, 2 and K's mean is 0
     StarRec *d_stars = nullptr;
     double *d_ep64 = nullptr;
@@ -543,8 +544,10 @@ extern "C" int joker_stars_create(joker_stars **out, int n_stars, int n_linear,
     s->max_epochs = max_ep;
     s->total_epochs = NE;
     s->off.assign(epoch_offsets, epoch_offsets + n_stars + 1);
-    for (int k = 0; k < n_stars; ++k)
+    for (int k = 0; k < n_stars; ++k) {
         s->fixed.push_back(fixed_flags(recs[k]));
+        s->epochs.push_back(recs[k].n_epochs);
+    }
     cudaError_t e = parts.allocate(s);
     if (e != cudaSuccess) {
         joker_stars_destroy(s);
@@ -583,6 +586,7 @@ extern "C" int joker_stars_create_slots(joker_stars **out, int n_slots, int max_
     s->total_epochs = (int64_t)n_slots * max_epochs;
     s->off.resize(n_slots + 1);
     s->fixed.assign(n_slots, 0);
+    s->epochs.assign(n_slots, 0);
     for (int k = 0; k <= n_slots; ++k) s->off[k] = (int64_t)k * max_epochs;
     std::vector<StarRec> recs(n_slots);
     memset(recs.data(), 0, sizeof(StarRec) * n_slots);
@@ -633,6 +637,7 @@ extern "C" int joker_stars_set(joker_stars *s, int slot, int n_epochs, const dou
                              sizeof(float) * r32.size(), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(s->d_stars + slot, &r, sizeof(StarRec), cudaMemcpyHostToDevice, st));
     s->fixed[slot] = fixed_flags(r);
+    s->epochs[slot] = n_epochs;
     // pageable sources: staged before the calls return
     return JOKER_OK;
 }
@@ -830,14 +835,20 @@ extern "C" int joker_cache_load(joker_cache *c, const double *d_chunk, int64_t n
 // ---------------------------------------------------------------- likelihood
 static int run_lnl(const joker_stars *s, int precision, LnlArgs a, int block,
                    cudaStream_t st) {
-    // the FP64 kernel takes its items by block
-    if (precision != JOKER_FP64) CUDA_TRY(cudaMemsetAsync(s->d_queue, 0, sizeof(int), st));
-    a.max_epochs = s->max_epochs;
-    // (a launch captured for other stars is right either way: both kernels take
-    // what the record lacks or has from the device)
-    a.doubles = 1;
-    for (int k = a.star0; k < a.star0 + a.n_sel && a.doubles; ++k)
-        a.doubles = !(s->fixed[k] & (s->jitter == JOKER_JITTER_APPLIED ? 2 : 1));
+    if (precision != JOKER_FP64) {
+        CUDA_TRY(cudaMemsetAsync(s->d_queue, 0, sizeof(int), st));
+    } else {                                     // its kernels take their items by block
+        // (a launch captured for other stars is right either way: both kernels
+        // take what a record has or lacks from the device)
+        a.doubles = 1;
+        int64_t sum = 0;
+        for (int k = a.star0; k < a.star0 + a.n_sel; ++k) {
+            if (s->fixed[k] & (s->jitter == JOKER_JITTER_APPLIED ? 2 : 1)) a.doubles = 0;
+            sum += s->epochs[k];
+            a.longest = std::max(a.longest, s->epochs[k]);
+        }
+        a.epochs = (int)(sum / std::max(a.n_sel, 1));
+    }
     CUDA_TRY(launch_lnl(precision, s->L, s->jitter == JOKER_JITTER_APPLIED, a, block, st));
     return JOKER_OK;
 }
@@ -887,7 +898,7 @@ void stars_internals(const joker_stars *s, const StarRec **recs, const double **
     *queue = s->d_queue;
 }
 
-int stars_max_epochs(const joker_stars *s) { return s->max_epochs; }
+int stars_epochs(const joker_stars *s, int star) { return s->epochs[star]; }
 // whether the star's records have the fixed-point form and its K prior mean is
 // zero, as that form's full system wants
 bool stars_fixed(const joker_stars *s, int star) { return (s->fixed[star] & 2) != 0; }

@@ -558,11 +558,25 @@ __device__ __forceinline__ bool sliced_epochs(AccFx<L, JIT> &acc, bool go, const
     return true;
 }
 
-// S for n samples of at most N epochs: four while the 128-sample blocks would
-// be fewer than four waves of the 608 that 152 SMs hold (a last wave of one
-// block in four costs most of a wave) and there are epochs to share out.
-inline int slices_for(int64_t n, int N) {
-    return n < 4 * 608 * 128 && N >= 16 ? 4 : 1;
+// S for n samples of N epochs (over several stars their mean, and the longest's)
+// on a GPU that holds `wave` blocks at a time.  Four warps share a sample's
+// epochs out but each makes the orbit's constants, worth some 4 epochs; they
+// gain while the samples alone leave SMs idle or a last wave short.  Times of
+// S = 4 over S = 1 (two linear parameters, six blocks an SM: 116736 samples a
+// wave):
+//   epochs   20000   60000   117000   160000   234000   311000 rows
+//     16      0.66    1.00     1.08     1.16     1.19     1.28
+//     40      0.58    0.91     0.95     1.00     1.03     1.10
+//    300      0.53    0.76     0.85     0.89
+// and likewise by waves with three blocks an SM: the line is N/32 waves, at most
+// four.  Beside shorter stars the longest one's chain is what S = 4 cuts, as long
+// as it outlasts the rest: seven stars of 3 epochs and one of 300, 50000 rows
+// each, 441 -> 326 us, eight of 3 to 250 449 -> 478 (left at S = 1).
+inline int slices_for(int64_t n, int N, int longest, int wave) {
+    const int64_t w = (int64_t)wave * SLICED_BLOCK;
+    const bool few = N >= 4 && 32 * n < N * w && n < 4 * w;
+    const bool chain = longest >= 4 && 5 * n * (N + 14) < 4 * longest * w;
+    return few || chain ? 4 : 1;
 }
 
 // FP64 ln L of one sample with the star's epochs read from global memory, in

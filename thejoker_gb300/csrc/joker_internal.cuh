@@ -11,6 +11,8 @@ constexpr int MAXL = JOKER_MAX_LINEAR;
 
 // Host-side count of the kernels this library has launched (joker_launch_count).
 void count_launch();
+// blocks of a kernel that the device holds at a time (cached)
+cudaError_t persistent_grid(const void *kern, int block, int *grid);
 constexpr int TILE = 256;          // epochs staged in shared memory at a time
 constexpr int REC32 = 20;          // floats per epoch record of the mixed kernel
 constexpr int REC64 = 16;          // doubles per FP64 epoch record: 8 doubles, then the
@@ -113,7 +115,7 @@ struct LnlArgs {
     int n_items;
     const int *n_items_dev;  // when set, the item count is read from device memory
     int star0, n_sel, chunk;
-    int max_epochs;          // of the table
+    int epochs, longest;     // FP64, implicit items: mean and most of the selected stars
     int doubles;             // FP64, implicit items: no star has the fixed-point form
     int64_t row0, count, ld, ips;
     const int *order;

@@ -160,8 +160,13 @@ static cudaError_t launch_fp64_LJ(LnlArgs a, cudaStream_t st) {
         // 310000 x 16: 652 -> 663)
         if (a.doubles)
             block = a.count * a.n_sel < 12 * 152 * SLICED_BLOCK ? 32 : SLICED_BLOCK;
-        else
-            S = slices_for(a.count * a.n_sel, a.max_epochs);
+        else {
+            int wave = 0;
+            const cudaError_t e = persistent_grid(
+                reinterpret_cast<const void *>(lnl_fp64_kernel<L, JIT>), SLICED_BLOCK, &wave);
+            if (e != cudaSuccess) return e;
+            S = slices_for(a.count * a.n_sel, a.epochs, a.longest, wave);
+        }
         const int64_t chunk = block / S, ips = (a.count + chunk - 1) / chunk;
         if (ips * a.n_sel <= INT32_MAX) {
             a.chunk = (int)chunk;

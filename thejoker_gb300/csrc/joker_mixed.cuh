@@ -767,8 +767,6 @@ lnl_mixed2_kernel(LnlArgs a) {
 // Persistent launch: as many CTAs as can be resident on the device (never more
 // than there are work items); each CTA loops over the shared work counter.
 // persistent_grid (joker_abi.cu) caches the grid per device, kernel and block.
-cudaError_t persistent_grid(const void *kern, int block, int *grid);
-
 template <typename K>
 inline cudaError_t launch_persistent(K kern, const LnlArgs &a, int block, cudaStream_t st) {
     int grid = 0;

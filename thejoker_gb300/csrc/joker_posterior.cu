@@ -434,11 +434,15 @@ cudaError_t launch_rv_elements(const double *t, int n_t, const double *el, int64
 
 template <int L, bool JIT>
 static cudaError_t launch_posterior_LJ(const StarRec *stars, const double *ep64, int star,
-                                       int max_epochs, const double *P, const double *E,
+                                       int epochs, const double *P, const double *E,
                                        const double *OM, const double *M0, const double *S,
                                        int64_t stride, const int64_t *rows, int64_t n, int k_clip,
                                        double *a, double *A, double *lnl, cudaStream_t st) {
-    const int sl = slices_for(n, max_epochs), per = SLICED_BLOCK / sl;
+    int wave = 0;
+    const cudaError_t e = persistent_grid(
+        reinterpret_cast<const void *>(posterior_kernel<L, JIT>), SLICED_BLOCK, &wave);
+    if (e != cudaSuccess) return e;
+    const int sl = slices_for(n, epochs, epochs, wave), per = SLICED_BLOCK / sl;
     const int64_t blocks = (n + per - 1) / per;
     if (blocks > INT32_MAX) return cudaErrorInvalidValue;
     posterior_kernel<L, JIT><<<(unsigned)blocks, SLICED_BLOCK, sliced_smem<L, JIT>(sl), st>>>(
@@ -450,16 +454,16 @@ static cudaError_t launch_posterior_LJ(const StarRec *stars, const double *ep64,
 // fixed: the star has a fixed-point form (stars_fixed).
 template <int L>
 static cudaError_t launch_posterior_L(const StarRec *stars, const double *ep64, int star,
-                                      bool fixed, int max_epochs, const double *P,
+                                      bool fixed, int epochs, const double *P,
                                       const double *E, const double *OM, const double *M0,
                                       const double *S, int64_t stride, const int64_t *rows,
                                       int64_t n, int jit, int k_clip, double *a, double *A,
                                       double *lnl, cudaStream_t st) {
     if (fixed && jit)
-        return launch_posterior_LJ<L, true>(stars, ep64, star, max_epochs, P, E, OM, M0, S, stride,
+        return launch_posterior_LJ<L, true>(stars, ep64, star, epochs, P, E, OM, M0, S, stride,
                                             rows, n, k_clip, a, A, lnl, st);
     if (fixed)
-        return launch_posterior_LJ<L, false>(stars, ep64, star, max_epochs, P, E, OM, M0, S, stride,
+        return launch_posterior_LJ<L, false>(stars, ep64, star, epochs, P, E, OM, M0, S, stride,
                                              rows, n, k_clip, a, A, lnl, st);
     const int64_t warps = n < 152 * 8 * 4 ? n : 152 * 8 * 4;
     const unsigned grid = (unsigned)((warps + 7) / 8);
@@ -470,13 +474,13 @@ static cudaError_t launch_posterior_L(const StarRec *stars, const double *ep64, 
 }
 
 cudaError_t launch_posterior(int L, const StarRec *stars, const double *ep64, int star,
-                             bool fixed, int max_epochs, const double *P, const double *E, const double *OM,
+                             bool fixed, int epochs, const double *P, const double *E, const double *OM,
                              const double *M0, const double *S, int64_t stride,
                              const int64_t *rows, int64_t n, int jit, int k_clip, double *a,
                              double *A, double *lnl, cudaStream_t st) {
     switch (L) {
 #define JOKER_POST_CASE(LL) \
-        case LL: return launch_posterior_L<LL>(stars, ep64, star, fixed, max_epochs, P, E, OM, M0, S, \
+        case LL: return launch_posterior_L<LL>(stars, ep64, star, fixed, epochs, P, E, OM, M0, S, \
                                                stride, rows, n, jit, k_clip, a, A, lnl, st);
         JOKER_POST_CASE(1) JOKER_POST_CASE(2) JOKER_POST_CASE(3)
         JOKER_POST_CASE(4) JOKER_POST_CASE(5) JOKER_POST_CASE(6)
@@ -502,7 +506,7 @@ namespace joker {
 void set_last_error(const char *msg);
 void stars_internals(const joker_stars *s, const StarRec **recs, const double **ep64,
                      const float **ep32, int *n_stars, int *L, int *jit, int **queue);
-int stars_max_epochs(const joker_stars *s);
+int stars_epochs(const joker_stars *s, int star);
 bool stars_fixed(const joker_stars *s, int star);
 void cache_internals(const joker_cache *c, int64_t *cap, const double **P, const double **E,
                      const double **OM, const double **M0, const double **S, int64_t *stride,
@@ -531,7 +535,7 @@ extern "C" int joker_linear_posterior(const joker_stars *stars, const joker_cach
     int64_t cap, stride; const double *P, *E, *OM, *M0, *S; const float4 *ma, *mb; const float *ms;
     cache_internals(cache, &cap, &P, &E, &OM, &M0, &S, &stride, &ma, &mb, &ms);
     const cudaError_t e = launch_posterior(L, recs, ep64, star, stars_fixed(stars, star),
-                                           stars_max_epochs(stars), P, E, OM, M0, S, stride, d_rows,
+                                           stars_epochs(stars, star), P, E, OM, M0, S, stride, d_rows,
                                            n, jit, k_clip, d_a, d_A, d_lnl, (cudaStream_t)stream);
     if (e != cudaSuccess) return post_fail(JOKER_ECUDA, cudaGetErrorString(e));
     return JOKER_OK;
