@@ -660,7 +660,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) accept_scan_kernel(AcceptArgs a)
 // on flag list 0 for re-evaluation in FP64 (or, past the list's capacity,
 // re-evaluated here), so that every ln L written out is within that of FP64.
 template <bool FLAG>
-__global__ void __launch_bounds__(ACC_THREADS) accept_emit_kernel(AcceptArgs a, int64_t total) {
+__global__ void __launch_bounds__(ACC_THREADS, 2) accept_emit_kernel(AcceptArgs a, int64_t total) {
     __shared__ int s_scan[ACC_THREADS];
     __shared__ int64_t s_block[ACC_THREADS];
     __shared__ int s_blocks;
