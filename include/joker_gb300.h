@@ -190,8 +190,10 @@ int joker_batch_marginal_ln_likelihood(const joker_stars *stars, int star,
  * bound on |lnL - lnL_FP64| per sample, and d_bound_key (optional, 2 per star)
  * the running maxima of lnL + err and lnL - err.
  * block (threads per CTA, 0 = 128) and chunk (samples per work item, a
- * multiple of block, 0 = 1024) tune the launch.  Calls that share one
- * joker_stars handle must be ordered on one stream. */
+ * multiple of block, 0 = 1024) tune the launch of the mixed precisions; at
+ * JOKER_FP64 they are checked, and the items are sized by the call (its rows,
+ * epochs and the kernel's occupancy).  Calls that share one joker_stars handle
+ * must be ordered on one stream. */
 int joker_lnl(const joker_stars *stars, const joker_cache *cache, int star0,
               int n_sel, int64_t row0, int64_t count, int precision,
               double *d_lnl, int64_t ld, uint64_t *d_max_key, float *d_err,

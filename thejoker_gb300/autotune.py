@@ -10,7 +10,8 @@ mode, the precision and the epoch counts, so it is measured: ``tune`` times
 events, after a warm-up launch) and records the fastest in a JSON table keyed
 by those properties.  ``chunk_for`` looks a workload up (default 1024 when it
 was never tuned); BatchRejection and IterativeBatch use it when no chunk is
-given.
+given.  (At "fp64" joker_lnl sizes its own items: every candidate launches alike,
+and the table's entry has no effect.)
 """
 import json
 import os
